@@ -135,6 +135,24 @@ void free_workspace(Workspace& ws) {
   ws.nmatmax = ws.ngkmax = ws.kmax = 0;
 }
 
+int handle_scratch(excfv_handle* h, size_t bytes, void** p) {
+  *p = nullptr;
+  if (bytes > h->scratch_bytes) {
+    if (h->scratch) cudaFree(h->scratch);
+    h->scratch = nullptr;
+    h->scratch_bytes = 0;
+    cudaError_t e = cudaMalloc(&h->scratch, bytes);
+    if (e != cudaSuccess) {
+      excfv_set_error("cudaMalloc of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
+      h->scratch = nullptr;
+      return EXCFV_ERR_ALLOC;
+    }
+    h->scratch_bytes = bytes;
+  }
+  *p = h->scratch;
+  return EXCFV_OK;
+}
+
 int stage_set_static(excfv_handle* h, const excfv_static* s) {
   DevStatic& st = h->st;
   h->static_gen++;
@@ -436,6 +454,7 @@ int excfv_destroy(excfv_handle* h) {
   free_rho(h->rho);
   free_sv(h->sv);
   if (h->kinfo) cudaFree(h->kinfo);
+  if (h->scratch) cudaFree(h->scratch);
   free_workspace(h->ws);
   if (h->owns_static) free_static(h->st);
   if (h->own_stream) cudaStreamDestroy(h->own_stream);

@@ -211,6 +211,10 @@ struct excfv_handle {
   double timings[4] = {0, 0, 0, 0};
   int nsm = 148;
   Prof prof;
+  // device scratch of the calls that upload host data and wait for their
+  // result (handle_scratch); grown to the largest call, freed with the handle
+  void* scratch = nullptr;
+  size_t scratch_bytes = 0;
   bool her2k_smem_set = false;  // k_her2k_f32's shared-memory limit raised on this device
 };
 
@@ -257,6 +261,9 @@ int potrf_diag_grouped(cudaStream_t s, const PotrfProb* d_probs, int nprob, int 
 
 // ---- stages (each enqueues work on h->stream) ------------------------------
 int stage_reserve(excfv_handle* h, int nmatmax, int ngkmax, int kmax);
+// `bytes` of the handle's scratch.  Only for calls that synchronise the stream
+// before they return: the next call, on whatever stream, takes the same memory.
+int handle_scratch(excfv_handle* h, size_t bytes, void** p);
 int stage_set_static(excfv_handle* h, const excfv_static* s);
 // genveffig / genmeffig on the device (interstitial.cu): kinds 0 veffig,
 // 1 meffig, 2 m2effig into dst[q] (device, ngvec), optional host copies

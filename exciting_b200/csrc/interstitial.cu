@@ -109,19 +109,17 @@ int stage_genfig(excfv_handle* h, const int* ngrid, const double* veffir, const 
       return EXCFV_ERR_ARG;
     }
   const long long N = (long long)n1 * n2 * n3;
-  double *d_v = nullptr, *d_c = nullptr;
-  cplx *z0 = nullptr, *z1 = nullptr;
+  void* base = nullptr;
+  if (int e0 = handle_scratch(h, (2 * sizeof(double) + 2 * sizeof(cplx)) * (size_t)N, &base)) return e0;
+  cplx *z0 = static_cast<cplx*>(base), *z1 = z0 + N;
+  double *d_v = reinterpret_cast<double*>(z1 + N), *d_c = d_v + N;
   int rc = EXCFV_OK;
   auto fail = [&](cudaError_t err) {
     excfv_set_error("genveffig: %s", cudaGetErrorString(err));
     rc = EXCFV_ERR_CUDA;
   };
   cudaError_t err;
-  if ((err = cudaMalloc(&d_v, sizeof(double) * N)) != cudaSuccess ||
-      (err = cudaMalloc(&d_c, sizeof(double) * N)) != cudaSuccess ||
-      (err = cudaMalloc(&z0, sizeof(cplx) * N)) != cudaSuccess ||
-      (err = cudaMalloc(&z1, sizeof(cplx) * N)) != cudaSuccess ||
-      (err = cudaMemcpyAsync(d_v, veffir, sizeof(double) * N, cudaMemcpyHostToDevice, s)) != cudaSuccess ||
+  if ((err = cudaMemcpyAsync(d_v, veffir, sizeof(double) * N, cudaMemcpyHostToDevice, s)) != cudaSuccess ||
       (err = cudaMemcpyAsync(d_c, cfunir, sizeof(double) * N, cudaMemcpyHostToDevice, s)) != cudaSuccess) {
     fail(err);
   } else {
@@ -152,10 +150,6 @@ int stage_genfig(excfv_handle* h, const int* ngrid, const double* veffir, const 
   }
   cudaError_t serr = cudaStreamSynchronize(s);
   if (rc == EXCFV_OK && serr != cudaSuccess) fail(serr);
-  cudaFree(d_v);
-  cudaFree(d_c);
-  cudaFree(z0);
-  cudaFree(z1);
   return rc;
 }
 
@@ -172,15 +166,13 @@ int stage_grid_field(excfv_handle* h, const int* ngrid, const double* f, const d
     return EXCFV_ERR_ARG;
   }
   const long long N = (long long)n1 * n2 * n3;
-  double *d_v = nullptr, *d_c = nullptr;
-  cplx *z0 = nullptr, *z1 = nullptr;
+  void* base = nullptr;
+  if (int e0 = handle_scratch(h, (2 * sizeof(double) + 2 * sizeof(cplx)) * (size_t)N, &base)) return e0;
+  cplx *z0 = static_cast<cplx*>(base), *z1 = z0 + N;
+  double *d_v = reinterpret_cast<double*>(z1 + N), *d_c = d_v + N;
   int rc = EXCFV_OK;
   cudaError_t err;
-  if ((err = cudaMalloc(&d_v, sizeof(double) * N)) != cudaSuccess ||
-      (err = cudaMalloc(&d_c, sizeof(double) * N)) != cudaSuccess ||
-      (err = cudaMalloc(&z0, sizeof(cplx) * N)) != cudaSuccess ||
-      (err = cudaMalloc(&z1, sizeof(cplx) * N)) != cudaSuccess ||
-      (err = cudaMemcpyAsync(d_v, f, sizeof(double) * N, cudaMemcpyHostToDevice, s)) != cudaSuccess ||
+  if ((err = cudaMemcpyAsync(d_v, f, sizeof(double) * N, cudaMemcpyHostToDevice, s)) != cudaSuccess ||
       (err = cudaMemcpyAsync(d_c, cfunir, sizeof(double) * N, cudaMemcpyHostToDevice, s)) != cudaSuccess) {
     excfv_set_error("interstitial field: %s", cudaGetErrorString(err));
     rc = EXCFV_ERR_CUDA;
@@ -204,9 +196,5 @@ int stage_grid_field(excfv_handle* h, const int* ngrid, const double* f, const d
     }
   }
   if (cudaStreamSynchronize(s) != cudaSuccess && rc == EXCFV_OK) rc = EXCFV_ERR_CUDA;
-  cudaFree(d_v);
-  cudaFree(d_c);
-  cudaFree(z0);
-  cudaFree(z1);
   return rc;
 }

@@ -554,8 +554,9 @@ int excfv_set_rho(excfv_handle* h, const excfv_rhoset* r) {
 }
 
 // G+k inputs of one k-point into the workspace; device or host pointers
+// (apwalm: also the matching coefficients in the reference layout)
 static int rho_stage_k(excfv_handle* h, int ngp, int ngkmax, int nmatmax, const double* gpc,
-                       const double* tpgpc, const double* sfacgp, cudaMemcpyKind kind) {
+                       const double* tpgpc, const double* sfacgp, cudaMemcpyKind kind, bool apwalm) {
   int rc;
   if ((rc = stage_reserve(h, nmatmax, ngkmax, std::max(1, h->st.nstfv)))) return rc;
   Workspace& ws = h->ws;
@@ -569,7 +570,7 @@ static int rho_stage_k(excfv_handle* h, int ngp, int ngkmax, int nmatmax, const 
   CUDA_TRY(cudaMemcpyAsync(ws.gpc, gpc, sizeof(double) * ngp, kind, s));
   CUDA_TRY(cudaMemcpyAsync(ws.tpgpc, tpgpc, sizeof(double) * 2 * ngp, kind, s));
   CUDA_TRY(cudaMemcpyAsync(ws.sfacgp, sfacgp, sizeof(cplx) * (size_t)ngkmax * h->st.natmtot, kind, s));
-  return stage_match(h, ngp, ngkmax, ws.apwalm);
+  return stage_match(h, ngp, ngkmax, apwalm ? ws.apwalm : nullptr);
 }
 
 static int check_rho(excfv_handle* h, int ngp, int ngkmax, int nmatmax) {
@@ -591,7 +592,7 @@ int excfv_rhovalk(excfv_handle* h, int32_t ngp, int32_t ngkmax, const double* gp
   if (rc) return rc;
   if (!gpc || !tpgpc || !sfacgp || !evecfv || !wocc) return EXCFV_ERR_ARG;
   DeviceGuard g(h->device);
-  if ((rc = rho_stage_k(h, ngp, ngkmax, nmatmax, gpc, tpgpc, sfacgp, cudaMemcpyHostToDevice))) return rc;
+  if ((rc = rho_stage_k(h, ngp, ngkmax, nmatmax, gpc, tpgpc, sfacgp, cudaMemcpyHostToDevice, !rho_packed(h)))) return rc;
   Workspace& ws = h->ws;
   // evecfv(nmatmax, nstfv) into the eigenvector scratch (nmatmax x kmax, kmax >= nstfv)
   const size_t need = (size_t)nmatmax * h->st.nstfv;
@@ -608,7 +609,7 @@ int excfv_rhovalk_dev(excfv_handle* h, int32_t ngp, int32_t ngkmax, const double
   if (rc) return rc;
   if (!gpc || !tpgpc || !sfacgp || !evecfv || !wocc) return EXCFV_ERR_ARG;
   DeviceGuard g(h->device);
-  if ((rc = rho_stage_k(h, ngp, ngkmax, nmatmax, gpc, tpgpc, sfacgp, cudaMemcpyDeviceToDevice))) return rc;
+  if ((rc = rho_stage_k(h, ngp, ngkmax, nmatmax, gpc, tpgpc, sfacgp, cudaMemcpyDeviceToDevice, !rho_packed(h)))) return rc;
   return stage_rhovalk(h, ngp, ngkmax, h->ws.apwalm, reinterpret_cast<const cplx*>(evecfv), nmatmax, wocc,
                        epsocc);
 }
@@ -721,7 +722,7 @@ static int rhovalk_sv_host(excfv_handle* h, bool nc, int32_t ngp, int32_t ngkmax
   if (rc) return rc;
   if (!gpc || !tpgpc || !sfacgp || !evecfv || !evecsv || !wocc) return EXCFV_ERR_ARG;
   DeviceGuard g(h->device);
-  if ((rc = rho_stage_k(h, ngp, ngkmax, nmatmax, gpc, tpgpc, sfacgp, cudaMemcpyHostToDevice))) return rc;
+  if ((rc = rho_stage_k(h, ngp, ngkmax, nmatmax, gpc, tpgpc, sfacgp, cudaMemcpyHostToDevice, true))) return rc;
   Workspace& ws = h->ws;
   const int n = h->st.nstfv;
   CUDA_TRY(cudaMemcpyAsync(ws.Z, evecfv, sizeof(cplx) * (size_t)nmatmax * n, cudaMemcpyHostToDevice, h->stream));

@@ -115,6 +115,9 @@ struct DevRho {
   cplx* zb = nullptr;
   double* rf = nullptr;
   double* rhomt = nullptr;
+  cplx* gang = nullptr;      // (states, radial functions of an atom, lmmaxvr, atoms of a group): states on the covering points
+  size_t gang_elems = 0;
+  double* rtp = nullptr;     // (nrcmax, lmmaxvr, natmtot) densities on the covering points
   cplx* coef = nullptr;
   double* w = nullptr;
   int* lo_first = nullptr;
@@ -271,6 +274,7 @@ int stage_genfig(excfv_handle* h, const int* ngrid, const double* veffir, const 
                  const int* kinds, cplx* const* dst, cplx* const* host_out);
 // muffin-tin valence density (rhoval.cu)
 int stage_set_rho(excfv_handle* h, const excfv_rhoset* r);
+bool rho_packed(const excfv_handle* h);  // the unpolarised density reads ws.Apk
 int stage_rhovalk(excfv_handle* h, int ngp, int ngkmax, const cplx* apwalm, const cplx* evec, long long ldev,
                   const double* wocc, double epsocc);
 int stage_rhovalk_sv(excfv_handle* h, int ngp, int ngkmax, const cplx* apwalm, const cplx* evec, long long ldev,

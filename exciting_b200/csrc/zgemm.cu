@@ -23,12 +23,12 @@
 #include "common.cuh"
 
 #include <algorithm>
+#include <cmath>
 #include <vector>
 
 namespace {
 
 constexpr int BM = 64, BN = 64, BK = 8, PAD = 4, NT = 128;
-constexpr int LDS = BM + PAD;
 
 __device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b) {
   asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
@@ -249,6 +249,157 @@ __global__ void __launch_bounds__(NT) zgemm_kernel(ZgemmArgs p) {
   zgemm_tile<OPA, OPB, BM>(p, i0, j0, bz, split, S);
 }
 
+// ---- small tiles: 32 x 32 outputs per CTA ---------------------------------
+// FP64 tensor work runs at 64 real FMAs per clock and SM, so a 64 x 64
+// tile keeps one SM busy for 256 clocks per unit of K and a product with few
+// tiles leaves most SMs idle: an order-316 product had 25 tiles (22.7 us).  With
+// 32 x 32 tiles it has 100.  A tile's products then take only 512 clocks per
+// k-tile, less than the latency of its loads, so the operands come through a
+// ring of four k-tiles filled by cp.async three ahead.  Elements stay
+// interleaved (one 16-byte copy each, zero-filled outside the matrix or the
+// triangle; conjugation is a sign in registers); rows of 32 + 2 elements keep
+// the fragment loads free of bank conflicts.  4 warps of 16 x 16 outputs.
+// Over one order-316 solve its 18 plain products went from 22.7 to 6.9 us each,
+// over an order-1964 one the products in all from 6.76 to 5.46 ms.
+constexpr int ST = 32, SPAD = 2, SSTG = 4;
+
+struct SmallSmem {
+  cplx A[SSTG][BK][ST + SPAD];
+  cplx B[SSTG][BK][ST + SPAD];
+};
+
+__device__ __forceinline__ void cp_async_el(cplx* dst, const cplx* src, bool ok) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(ok ? 16 : 0) : "memory");
+}
+
+template <int OPA, int OPB>
+__global__ void __launch_bounds__(128) zgemm_small_kernel(ZgemmArgs p) {
+  __shared__ __align__(16) SmallSmem S;
+  const bool rev_x = p.tri_a == TRI_LOWER;
+  const bool rev_y = p.tri_b == TRI_UPPER || (p.tri_a == TRI_LOWER && p.uplo_c == TRI_UPPER);
+  const int i0 = (rev_x ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x) * ST;
+  const int j0 = (rev_y ? (int)(gridDim.y - 1 - blockIdx.y) : (int)blockIdx.y) * ST;
+  if (p.uplo_c == TRI_UPPER && i0 > j0 + ST - 1) return;
+  if (p.uplo_c == TRI_LOWER && j0 > i0 + ST - 1) return;
+  const long long bz = blockIdx.z / p.splitk;
+  const int split = (int)(blockIdx.z % p.splitk);
+  const cplx* __restrict__ A = p.A + bz * p.strideA;
+  const cplx* __restrict__ B = p.B + bz * p.strideB;
+  cplx* __restrict__ C = p.C + bz * p.strideC;
+  int kbeg = 0, kend = p.k - p.kdec * (int)bz;
+  if (p.tri_a == TRI_LOWER) kend = min(kend, i0 + ST);
+  if (p.tri_a == TRI_UPPER) kbeg = max(kbeg, i0);
+  if (p.tri_b == TRI_UPPER) kend = min(kend, j0 + ST);
+  if (p.tri_b == TRI_LOWER) kbeg = max(kbeg, j0);
+  kbeg = (kbeg / BK) * BK;
+  if (p.splitk > 1 && kend > kbeg) {
+    const int chunk = ((kend - kbeg + p.splitk - 1) / p.splitk + BK - 1) / BK * BK;
+    kbeg += split * chunk;
+    kend = min(kend, kbeg + chunk);
+  }
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int wm = (warp & 1) * 16, wn = (warp >> 1) * 16;
+  const int nk = (kend > kbeg) ? (kend - kbeg + BK - 1) / BK : 0;
+
+  auto issue = [&](int kt) {
+    if (kt < nk) {
+      const int st = kt % SSTG, k0 = kbeg + kt * BK;
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const int idx = tid + r * 128;
+        int ii, kk;
+        if (OPA == OP_N) { ii = idx & 31; kk = idx >> 5; }
+        else { kk = idx & 7; ii = idx >> 3; }
+        const int gi = i0 + ii, gk = k0 + kk;
+        bool ok = gi < p.m && gk < kend;
+        if (p.tri_a == TRI_LOWER && gk > gi) ok = false;
+        if (p.tri_a == TRI_UPPER && gk < gi) ok = false;
+        const cplx* src = (OPA == OP_N) ? A + gi + (long long)gk * p.lda : A + gk + (long long)gi * p.lda;
+        cp_async_el(&S.A[st][kk][ii], ok ? src : A, ok);
+      }
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const int idx = tid + r * 128;
+        int jj, kk;
+        if (OPB == OP_N) { kk = idx & 7; jj = idx >> 3; }
+        else { jj = idx & 31; kk = idx >> 5; }
+        const int gj = j0 + jj, gk = k0 + kk;
+        bool ok = gj < p.n && gk < kend;
+        if (p.tri_b == TRI_UPPER && gk > gj) ok = false;
+        if (p.tri_b == TRI_LOWER && gk < gj) ok = false;
+        const cplx* src = (OPB == OP_N) ? B + gk + (long long)gj * p.ldb : B + gj + (long long)gk * p.ldb;
+        cp_async_el(&S.B[st][kk][jj], ok ? src : B, ok);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+
+  double acc[2][2][2][2];
+#pragma unroll
+  for (int a = 0; a < 2; ++a)
+#pragma unroll
+    for (int b = 0; b < 2; ++b)
+#pragma unroll
+      for (int c = 0; c < 2; ++c) acc[a][b][c][0] = acc[a][b][c][1] = 0.0;
+#pragma unroll
+  for (int q = 0; q < SSTG - 1; ++q) issue(q);
+  const int cc = lane >> 2;
+  for (int kt = 0; kt < nk; ++kt) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(SSTG - 2) : "memory");
+    __syncthreads();          // tile kt has landed; tile kt-1's slot is free
+    issue(kt + SSTG - 1);
+    const int st = kt % SSTG;
+#pragma unroll
+    for (int ks = 0; ks < BK; ks += 4) {
+      const int kr = ks + (lane & 3);
+      cplx av[2], bv[2];
+#pragma unroll
+      for (int t = 0; t < 2; ++t) {
+        av[t] = S.A[st][kr][wm + t * 8 + cc];
+        bv[t] = S.B[st][kr][wn + t * 8 + cc];
+        if (OPA == OP_C) av[t].y = -av[t].y;
+        if (OPB == OP_C) bv[t].y = -bv[t].y;
+      }
+#pragma unroll
+      for (int a = 0; a < 2; ++a)
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+          dmma(acc[a][b][0][0], acc[a][b][0][1], av[a].x, bv[b].x);
+          dmma(acc[a][b][1][0], acc[a][b][1][1], av[a].x, bv[b].y);
+          dmma(acc[a][b][0][0], acc[a][b][0][1], av[a].y, -bv[b].y);
+          dmma(acc[a][b][1][0], acc[a][b][1][1], av[a].y, bv[b].x);
+        }
+    }
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  const bool use_beta = (p.beta.x != 0.0 || p.beta.y != 0.0);
+  cplx* P = p.part + ((long long)split * p.batch + bz) * (long long)p.m * p.n;
+#pragma unroll
+  for (int a = 0; a < 2; ++a) {
+    const int row = i0 + wm + a * 8 + (lane >> 2);
+    if (row >= p.m) continue;
+#pragma unroll
+    for (int b = 0; b < 2; ++b)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int col = j0 + wn + b * 8 + (lane & 3) * 2 + e;
+        if (col >= p.n) continue;
+        const cplx v = cmk(acc[a][b][0][e], acc[a][b][1][e]);
+        if (p.splitk > 1) {
+          P[row + (long long)col * p.m] = v;
+          continue;
+        }
+        if (p.uplo_c == TRI_UPPER && row > col) continue;
+        if (p.uplo_c == TRI_LOWER && row < col) continue;
+        cplx out = cmul(p.alpha, v);
+        cplx* dst = C + row + (long long)col * p.ldc;
+        if (use_beta) out = cadd(out, cmul(p.beta, *dst));
+        *dst = out;
+      }
+  }
+}
+
 // Grouped form: one launch over the TBM x 64 tiles of many independent
 // products of different sizes.  tiles[b] = (problem, row tile, column tile, -) of CTA b,
 // listed by the host heaviest first; probs[problem] is an unbatched product
@@ -281,9 +432,11 @@ __global__ void k_splitk_reduce(ZgemmArgs p) {
 }
 
 template <int OPA, int OPB>
-int launch(cudaStream_t s, const ZgemmArgs& a) {
-  dim3 grid((a.m + BM - 1) / BM, (a.n + BN - 1) / BN, a.batch * max(1, a.splitk));
-  zgemm_kernel<OPA, OPB><<<grid, NT, 0, s>>>(a); count_launch();
+int launch(cudaStream_t s, const ZgemmArgs& a, int tile) {
+  dim3 grid((a.m + tile - 1) / tile, (a.n + tile - 1) / tile, a.batch * max(1, a.splitk));
+  if (tile == ST) zgemm_small_kernel<OPA, OPB><<<grid, 128, 0, s>>>(a);
+  else zgemm_kernel<OPA, OPB><<<grid, NT, 0, s>>>(a);
+  count_launch();
   if (a.splitk > 1) {
     const long long tot = (long long)a.m * a.n * a.batch;
     k_splitk_reduce<<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(a); count_launch();
@@ -302,36 +455,54 @@ int zgemm(cudaStream_t s, int opA, int opB, const ZgemmArgs& a_in) {
   ZgemmArgs a = a_in;
   if (a.m <= 0 || a.n <= 0 || a.batch <= 0) return 0;
   if (a.k <= 0 && a.beta.x == 1.0 && a.beta.y == 0.0) return 0;
-  // split-K when the output has too few tiles to fill the GPU and K is long
+  // The tile (64 or 32) and the number of K pieces with the shortest estimated
+  // time: rounds of CTAs over the SMs times a CTA's clocks (tile^2 / 16 per unit
+  // of K, a tenth more for 32 x 32 tiles, which load twice as much per product,
+  // plus a start of 3000), and for split K the reduction's launch and traffic.
+  // A large product always gets 64 x 64 tiles and one piece.  Products in place
+  // (a panel overwritten by its own product) need one CTA per column of tiles:
+  // 64-row tiles, no pieces.
   a.splitk = 1;
   a.part = nullptr;
+  int tile = BM;
+  const bool in_place = (a.B == a.C) || (a.A == a.C);
   {
-    const long long tm = (a.m + BM - 1) / BM, tn = (a.n + BN - 1) / BN;
-    long long tiles = tm * tn * a.batch;
-    if (a.uplo_c != TRI_NONE && a.m == a.n) tiles = (tiles + tm * a.batch) / 2;
-    const int nsm = g_ctx.nsm;
-    if (g_ctx.ws && tiles < nsm && a.k >= 256) {
-      int sk = (int)((2 * nsm + tiles - 1) / tiles);
-      sk = min(sk, a.k / 128);
-      sk = min(sk, 32);
-      const long long need = (long long)a.m * a.n * a.batch;
-      while (sk > 1 && (size_t)(need * sk) > g_ctx.cap) --sk;
-      if (sk > 1) {
-        a.splitk = sk;
-        a.part = g_ctx.ws;
+    const double nsm = g_ctx.nsm;
+    double best = 1e300;
+    for (int t : {BM, ST}) {
+      if (in_place && t != BM) break;
+      const long long tm = (a.m + t - 1) / t, tn = (a.n + t - 1) / t;
+      long long tiles = tm * tn * a.batch;
+      if (a.uplo_c != TRI_NONE && a.m == a.n) tiles = (tiles + tm * a.batch) / 2;
+      if (t == BM && tiles >= 4 * (long long)g_ctx.nsm) break;  // a large product
+      const double per_k = t * t / 16.0 * (t == ST ? 1.1 : 1.0);
+      for (int sk : {1, 2, 3, 4, 6, 8, 12, 16, 24, 32}) {
+        if (sk > 1 && (in_place || !g_ctx.ws || a.k < 32 * sk)) break;
+        const long long need = (long long)a.m * a.n * a.batch * sk;
+        if (sk > 1 && (size_t)need > g_ctx.cap) break;
+        const double ctas = (double)tiles * sk;
+        const double rounds = std::max(1.0, std::ceil(ctas / nsm));
+        double est = rounds * ((double)a.k / sk) * per_k + 3000.0;
+        if (sk > 1) est += 5000.0 + 32.0 * need / 2000.0;
+        if (est < 0.95 * best) {
+          best = est;
+          tile = t;
+          a.splitk = sk;
+        }
       }
     }
+    if (a.splitk > 1) a.part = g_ctx.ws;
   }
   switch (opA * 3 + opB) {
-    case OP_N * 3 + OP_N: return launch<OP_N, OP_N>(s, a);
-    case OP_N * 3 + OP_C: return launch<OP_N, OP_C>(s, a);
-    case OP_N * 3 + OP_T: return launch<OP_N, OP_T>(s, a);
-    case OP_C * 3 + OP_N: return launch<OP_C, OP_N>(s, a);
-    case OP_C * 3 + OP_C: return launch<OP_C, OP_C>(s, a);
-    case OP_C * 3 + OP_T: return launch<OP_C, OP_T>(s, a);
-    case OP_T * 3 + OP_N: return launch<OP_T, OP_N>(s, a);
-    case OP_T * 3 + OP_C: return launch<OP_T, OP_C>(s, a);
-    case OP_T * 3 + OP_T: return launch<OP_T, OP_T>(s, a);
+    case OP_N * 3 + OP_N: return launch<OP_N, OP_N>(s, a, tile);
+    case OP_N * 3 + OP_C: return launch<OP_N, OP_C>(s, a, tile);
+    case OP_N * 3 + OP_T: return launch<OP_N, OP_T>(s, a, tile);
+    case OP_C * 3 + OP_N: return launch<OP_C, OP_N>(s, a, tile);
+    case OP_C * 3 + OP_C: return launch<OP_C, OP_C>(s, a, tile);
+    case OP_C * 3 + OP_T: return launch<OP_C, OP_T>(s, a, tile);
+    case OP_T * 3 + OP_N: return launch<OP_T, OP_N>(s, a, tile);
+    case OP_T * 3 + OP_C: return launch<OP_T, OP_C>(s, a, tile);
+    case OP_T * 3 + OP_T: return launch<OP_T, OP_T>(s, a, tile);
   }
   return EXCFV_ERR_ARG;
 }

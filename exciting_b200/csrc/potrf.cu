@@ -16,126 +16,138 @@ namespace {
 
 constexpr int NBP = 64;
 
-// One CTA of 32 x 32 threads factors the b x b diagonal block (b <= 64) and
-// inverts the factor, as a 2 x 2 block recursion on 32 x 32 blocks held in
-// shared memory (thread (r, c) owns element (r, c) of a 32-block):
-//   U11 = chol(A11), X11 = U11^-1, U12 = X11^H A12, A22 -= U12^H U12,
-//   U22 = chol(A22), X22 = U22^-1, X12 = -X11 U12 X22.
-// FP64 vector throughput bounds this kernel, so the work is laid out such
-// that whole warps (one row each) drop out of every elimination step.
-// Rows/columns past b are padded with the identity.
+// One CTA factors the b x b diagonal block (b <= 64) and inverts the factor: a
+// right-looking elimination of [A | I] in steps of four columns, which leaves
+// U = L^H in A and L^-1 = (U^-1)^H in the unit part.  Per step
+//   the two warps that own the 64 active columns (A's columns right of the
+//   step, the unit part's up to it) each factor the 4 x 4 diagonal block
+//   redundantly in registers and solve their own column's four entries;
+//   --- barrier ---
+//   every warp updates four rows at a time with the four pivot rows;
+//   --- barrier ---
+// so 16 steps cost 32 barriers and a chain of four rsqrt each.  Bound by that
+// chain and by shared-memory traffic (four rows share each pivot-row load).
+// A 64-block takes 30 us and a 22-block 15; a column at a time with 1024 threads
+// and ~260 barriers took 57 us for either.
 constexpr int LDB = 65;
+constexpr int DT = 512;
 
-__device__ __forceinline__ bool chol32(cplx* A, double* rinv, int o, int tr, int tc, int* s_fail, int fail_base) {
-  // A is the 64 x LDB shared block; factor A(o:o+32, o:o+32) in place (upper)
-  if (tr == 0 && tc == 0) {
-    const double a = A[o * LDB + o].x;
-    rinv[o] = (a > 0.0) ? 1.0 / sqrt(a) : 0.0;
-    if (!(a > 0.0)) *s_fail = fail_base + 1;
+// Cholesky of the Hermitian 4 x 4 block at A(j, j) (upper part read): u above
+// the diagonal, r = 1 / U(k, k).  Returns 0, or the 1-based first pivot that
+// is not positive.
+__device__ __forceinline__ int chol4(const cplx* A, int j, cplx (&u)[4][4], double (&r)[4]) {
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+#pragma unroll
+    for (int c = k; c < 4; ++c) u[k][c] = A[(j + k) * LDB + j + c];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const double d = u[k][k].x;
+    if (!(d > 0.0)) return k + 1;
+    r[k] = 1.0 / sqrt(d);
+#pragma unroll
+    for (int c = k; c < 4; ++c) u[k][c] = (c == k) ? cmk(d * r[k], 0.0) : cscale(u[k][c], r[k]);
+#pragma unroll
+    for (int k2 = k + 1; k2 < 4; ++k2)
+#pragma unroll
+      for (int c = k2; c < 4; ++c) u[k2][c] = csub(u[k2][c], cmulc(u[k][k2], u[k][c]));
   }
-  __syncthreads();
-  for (int j = 0; j < 32; ++j) {
-    if (*s_fail) return false;
-    if (tr == j && tc >= j) A[(o + j) * LDB + o + tc] = cscale(A[(o + j) * LDB + o + tc], rinv[o + j]);
-    __syncthreads();
-    if (tr > j && tc >= tr) {
-      cplx* x = &A[(o + tr) * LDB + o + tc];
-      *x = csub(*x, cmulc(A[(o + j) * LDB + o + tr], A[(o + j) * LDB + o + tc]));
-      if (tr == j + 1 && tc == j + 1) {
-        const double a = x->x;
-        rinv[o + j + 1] = (a > 0.0) ? 1.0 / sqrt(a) : 0.0;
-        if (!(a > 0.0)) *s_fail = fail_base + j + 2;
-      }
-    }
-    __syncthreads();
-  }
-  return true;
-}
-
-// X(o:o+32, o:o+32) = inverse of the upper factor U(o:o+32, o:o+32)
-__device__ __forceinline__ void inv32(const cplx* A, cplx* X, const double* rinv, int o, int tr, int tc) {
-  X[(o + tr) * LDB + o + tc] = cmk(tr == tc ? 1.0 : 0.0, 0.0);
-  __syncthreads();
-  for (int i = 31; i >= 0; --i) {
-    if (tr == i && tc >= i) X[(o + i) * LDB + o + tc] = cscale(X[(o + i) * LDB + o + tc], rinv[o + i]);
-    __syncthreads();
-    if (tr < i && tc >= i)
-      X[(o + tr) * LDB + o + tc] = csub(X[(o + tr) * LDB + o + tc],
-                                        cmul(A[(o + tr) * LDB + o + i], X[(o + i) * LDB + o + tc]));
-    __syncthreads();
-  }
+  return 0;
 }
 
 __device__ __forceinline__ void potrf_diag_block(int n, int kb, cplx* O, long long ld, cplx* Ui, int* status) {
   extern __shared__ __align__(16) unsigned char dsm[];
   cplx* A = reinterpret_cast<cplx*>(dsm);   // 64 x LDB, row-major [r][c]
-  cplx* X = A + NBP * LDB;
-  __shared__ double rinv[NBP];
+  cplx* Y = A + NBP * LDB;                  // the unit part, L^-1 at the end
   __shared__ int s_fail;
   if (status[ST_POTRF] != 0) return;
   const int b = min(NBP, n - kb);
-  const int tc = threadIdx.x & 31, tr = threadIdx.x >> 5;
-  for (int t = threadIdx.x; t < NBP * NBP; t += 1024) {
+  const int lim = (b + 3) / 4 * 4;          // rows past b are padded with the identity
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int t = tid; t < NBP * NBP; t += DT) {
     const int r = t % NBP, c = t / NBP;  // coalesced along r
     cplx a = cmk(r == c ? 1.0 : 0.0, 0.0);
+    Y[r * LDB + c] = a;
     if (r < b && c < b && r <= c) a = O[(kb + r) + ld * (kb + c)];
+    if (r == c) a.y = 0.0;
     A[r * LDB + c] = a;
-    X[r * LDB + c] = cmk(0.0, 0.0);
   }
-  if (threadIdx.x == 0) s_fail = 0;
+  if (tid == 0) s_fail = 0;
   __syncthreads();
-  if (!chol32(A, rinv, 0, tr, tc, &s_fail, 0)) {
-    if (threadIdx.x == 0 && s_fail <= b) atomicCAS(&status[ST_POTRF], 0, kb + s_fail);
-    return;
-  }
-  inv32(A, X, rinv, 0, tr, tc);
-  // U12 = X11^H A12 (thread (r, c): column 32 + c)
-  {
-    cplx acc = cmk(0.0, 0.0);
-    for (int k = 0; k <= tr; ++k) acc = cadd(acc, cmulc(X[k * LDB + tr], A[k * LDB + 32 + tc]));
+  for (int j = 0; j < lim; j += 4) {
+    cplx u[4][4];
+    double r[4];
+    if (tid < 64) {
+      const int bad = chol4(A, j, u, r);
+      if (bad) {
+        if (tid == 0) s_fail = j + bad;
+      } else {
+        // columns right of the step in A, then columns 0 .. j + 3 of the unit part
+        const bool inA = tid < 60 - j;
+        cplx* col = inA ? A + j + 4 + tid : Y + tid - (60 - j);
+        cplx x[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          x[k] = col[(j + k) * LDB];
+#pragma unroll
+          for (int q = 0; q < k; ++q) x[k] = csub(x[k], cmulc(u[q][k], x[q]));
+          x[k] = cscale(x[k], r[k]);
+          col[(j + k) * LDB] = x[k];
+        }
+      }
+    }
     __syncthreads();
-    A[tr * LDB + 32 + tc] = acc;
+    if (s_fail) {
+      if (tid == 0 && s_fail <= b) atomicCAS(&status[ST_POTRF], 0, kb + s_fail);
+      return;
+    }
+    if (tid == 0) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+#pragma unroll
+        for (int c = k; c < 4; ++c) A[(j + k) * LDB + j + c] = u[k][c];
+    }
+    // rows i = j + 4 + warp + 16 q of both parts: row -= sum_k conj(U(j+k, i)) (row j+k)
+    const int i0 = j + 4 + warp;
+    if (i0 < lim) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int c = lane + 32 * h;
+        const bool inA = c >= j + 4;
+        cplx* M = inA ? A : Y;
+        if (c >= lim) continue;
+        cplx pv[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) pv[k] = M[(j + k) * LDB + c];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const int i = i0 + 16 * q;
+          if (i >= lim || (inA && c < i)) continue;
+          cplx v = M[i * LDB + c];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) v = csub(v, cmulc(A[(j + k) * LDB + i], pv[k]));
+          M[i * LDB + c] = v;
+        }
+      }
+    }
     __syncthreads();
   }
-  // A22 -= U12^H U12 (upper)
-  if (tc >= tr) {
-    cplx acc = cmk(0.0, 0.0);
-    for (int k = 0; k < 32; ++k) acc = cadd(acc, cmulc(A[k * LDB + 32 + tr], A[k * LDB + 32 + tc]));
-    A[(32 + tr) * LDB + 32 + tc] = csub(A[(32 + tr) * LDB + 32 + tc], acc);
-  }
-  __syncthreads();
-  if (!chol32(A, rinv, 32, tr, tc, &s_fail, 32)) {
-    if (threadIdx.x == 0 && s_fail <= b) atomicCAS(&status[ST_POTRF], 0, kb + s_fail);
-    return;
-  }
-  inv32(A, X, rinv, 32, tr, tc);
-  // X12 = -X11 (U12 X22): T = U12 X22 into X's lower-left block, then X12
-  {
-    cplx acc = cmk(0.0, 0.0);
-    for (int k = 0; k <= tc; ++k) acc = cadd(acc, cmul(A[tr * LDB + 32 + k], X[(32 + k) * LDB + 32 + tc]));
-    X[(32 + tr) * LDB + tc] = acc;  // scratch: lower-left block of X
-    __syncthreads();
-    cplx acc2 = cmk(0.0, 0.0);
-    for (int k = tr; k < 32; ++k) acc2 = cadd(acc2, cmul(X[tr * LDB + k], X[(32 + k) * LDB + tc]));
-    X[tr * LDB + 32 + tc] = cmk(-acc2.x, -acc2.y);
-    __syncthreads();
-  }
-  for (int t = threadIdx.x; t < NBP * NBP; t += 1024) {
+  for (int t = tid; t < NBP * NBP; t += DT) {
     const int r = t % NBP, c = t / NBP;
     if (r < b && c < b && r <= c) {
       O[(kb + r) + ld * (kb + c)] = A[r * LDB + c];
-      Ui[(kb + r) + ld * (kb + c)] = X[r * LDB + c];
+      Ui[(kb + r) + ld * (kb + c)] = cconj(Y[c * LDB + r]);
     }
   }
 }
 
-__global__ void __launch_bounds__(1024) k_potrf_diag(int n, int kb, cplx* O, long long ld, cplx* Ui,
-                                                     int* status) {
+__global__ void __launch_bounds__(DT) k_potrf_diag(int n, int kb, cplx* O, long long ld, cplx* Ui,
+                                                   int* status) {
   potrf_diag_block(n, kb, O, ld, Ui, status);
 }
 
 // Grouped form: CTA b factors diagonal block kb of problem b.
-__global__ void __launch_bounds__(1024) k_potrf_diag_grouped(const PotrfProb* __restrict__ probs, int kb) {
+__global__ void __launch_bounds__(DT) k_potrf_diag_grouped(const PotrfProb* __restrict__ probs, int kb) {
   const PotrfProb p = probs[blockIdx.x];
   potrf_diag_block(p.n, kb, p.O, p.ld, p.Ui, p.status);
 }
@@ -149,7 +161,7 @@ int potrf_diag_grouped(cudaStream_t s, const PotrfProb* d_probs, int nprob, int 
   if (nprob <= 0) return EXCFV_OK;
   const int smem = potrf_smem_bytes();
   CUDA_TRY(cudaFuncSetAttribute(k_potrf_diag_grouped, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  k_potrf_diag_grouped<<<nprob, 1024, smem, s>>>(d_probs, kb); count_launch();
+  k_potrf_diag_grouped<<<nprob, DT, smem, s>>>(d_probs, kb); count_launch();
   CUDA_TRY(cudaGetLastError());
   return EXCFV_OK;
 }
@@ -161,7 +173,7 @@ int potrf_upper(excfv_handle* h, int n, cplx* O, cplx* Ui, long long ld) {
   CUDA_TRY(cudaFuncSetAttribute(k_potrf_diag, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   for (int kb = 0; kb < n; kb += NBP) {
     const int b = min(NBP, n - kb);
-    k_potrf_diag<<<1, 1024, smem, s>>>(n, kb, O, ld, Ui, h->ws.status); count_launch();
+    k_potrf_diag<<<1, DT, smem, s>>>(n, kb, O, ld, Ui, h->ws.status); count_launch();
     CUDA_TRY(cudaGetLastError());
     const int rest = n - kb - b;
     if (rest <= 0) break;

@@ -16,6 +16,7 @@ int mirror_upper(cudaStream_t s, int n, cplx* M, long long ld);
 size_t tridiag_eig_scratch_doubles(int n, int k);
 int tridiag_workspace_doubles();
 int tridiag_nb();
+size_t tridiag_flow_bytes(int n, int nsm);
 
 namespace {
 thread_local char g_err[512] = "";
@@ -126,7 +127,9 @@ void free_workspace(Workspace& ws) {
   dfree(ws.tpgpc); dfree(ws.sfacgp); dfree(ws.gk_iv); dfree(ws.d); dfree(ws.e); dfree(ws.tau);
   dfree(ws.Wp); dfree(ws.red); dfree(ws.w); dfree(ws.stein_ws); dfree(ws.icl); dfree(ws.ybuf);
   dfree(ws.Z); dfree(ws.Z2); dfree(ws.Gk); dfree(ws.Gki); dfree(ws.Tf); dfree(ws.Xs);
-  dfree(ws.status); dfree(ws.bar); dfree(ws.part); dfree(ws.prog); dfree(ws.slices); dfree(ws.slice_sc);
+  dfree(ws.status); dfree(ws.bar); dfree(ws.part); dfree(ws.prog);
+  if (ws.flow) cudaFree(ws.flow);
+  ws.flow = nullptr; dfree(ws.slices); dfree(ws.slice_sc);
   ws.slices_elems = ws.slice_sc_n = 0;
   if (ws.h_pinned) cudaFreeHost(ws.h_pinned);
   ws.h_pinned = nullptr;
@@ -373,6 +376,7 @@ int stage_reserve(excfv_handle* h, int nmatmax, int ngkmax, int kmax) {
       (rc = dalloc(&ws.Tf, backtr_factor_elems((int)n))) || (rc = dalloc(&ws.Xs, 2 * 256 * K)) ||
       (rc = dalloc(&ws.status, (size_t)ST_NWORDS)) || (rc = dalloc(&ws.bar, (size_t)4)) ||
       (rc = dalloc(&ws.prog, n)) ||
+      (rc = dalloc(reinterpret_cast<unsigned char**>(&ws.flow), tridiag_flow_bytes((int)n, h->nsm))) ||
       (rc = dalloc(&ws.part, std::max((size_t)(8u << 20), n * 64 * 4)))) {
     free_workspace(ws);
     return rc;

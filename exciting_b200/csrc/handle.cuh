@@ -92,6 +92,7 @@ struct Workspace {
   size_t part_cap = 0;      // complex elements
   int* status = nullptr;    // ST_NWORDS
   unsigned int* bar = nullptr;  // grid barrier words
+  void* flow = nullptr;     // words of the dataflow panel kernel (tridiag_flow.cu)
   int* prog = nullptr;      // (n) per-sweep progress of the band -> tridiagonal chase
   // split-BF16 setup of the precision form: slice planes of A and of aa A, row scales
   __nv_bfloat16* slices = nullptr;

@@ -29,35 +29,13 @@
 // bounded in time; a timeout sets status[ST_BARRIER] and every CTA then
 // leaves the kernel.  The kernel is instantiated for FP64 storage and for
 // complex64 storage (the precision form), with FP64 reflector arithmetic.
-#include <cuda.h>
-#include <cudaTypedefs.h>
-
-#include "handle.cuh"
+#include "tridiag_dev.cuh"
 
 namespace {
 
-constexpr int NBT = 32;
 constexpr int TT = 256;
-constexpr int RCH = 64;
 constexpr int MAXCH = 2;   // row chunks per CTA held in shared memory (FP64 storage)
 constexpr int MAXCH_C64 = 3;  // complex64 storage: up to three, for more concurrent lanes
-
-// Storage type T2 of C, V and W: double2 (FP64 form) or float2 (the precision
-// form's complex64 copy).  Arithmetic is FP64 in both.
-__device__ __forceinline__ cplx ldT(const double2* p) { return __ldcg(p); }
-__device__ __forceinline__ cplx ldT(const float2* p) {
-  const float2 v = __ldcg(p);
-  return cmk((double)v.x, (double)v.y);
-}
-__device__ __forceinline__ void stT(double2* p, cplx v) { *p = v; }
-__device__ __forceinline__ void stT(float2* p, cplx v) { *p = make_float2((float)v.x, (float)v.y); }
-__device__ __forceinline__ cplx toD(double2 v) { return v; }
-__device__ __forceinline__ cplx toD(float2 v) { return cmk((double)v.x, (double)v.y); }
-template <typename T2> __device__ __forceinline__ T2 fromD(cplx v);
-template <> __device__ __forceinline__ double2 fromD<double2>(cplx v) { return v; }
-template <> __device__ __forceinline__ float2 fromD<float2>(cplx v) {
-  return make_float2((float)v.x, (float)v.y);
-}
 
 template <typename T2, int MC>
 struct PanelSmem {
@@ -66,24 +44,11 @@ struct PanelSmem {
   cplx X[MC][RCH];
 };
 
-__device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
-  unsigned v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ long long gtimer() {
-  long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-__device__ __forceinline__ cplx ldc(const cplx* p) { return __ldcg(p); }
-__device__ __forceinline__ double ldd(const double* p) { return __ldcg(p); }
-
 // Tiles of the trailing matrix for y = C22 v: 64 rows x BC columns (16 KB),
 // streamed through a ring of STAGES shared-memory slots by TMA.
 template <typename T2, int MC>
 struct Ring {
-  static constexpr int BC = (sizeof(T2) == 16) ? 16 : 32;
+  static constexpr int BC = TILE_COLS<T2>;
   static constexpr int STAGES = (sizeof(T2) == 16) ? (MC == 1 ? 8 : 4) : (MC <= 2 ? 8 : 6);
   static constexpr int TILE = RCH * BC;  // elements
   static constexpr unsigned BYTES = TILE * sizeof(T2);
@@ -95,92 +60,8 @@ constexpr size_t panel_smem_bytes() {
   return sizeof(PanelSmem<T2, MC>) + 128 + (size_t)Ring<T2, MC>::STAGES * Ring<T2, MC>::BYTES;
 }
 
-__device__ __forceinline__ unsigned smem_u32(const void* p) {
-  return (unsigned)__cvta_generic_to_shared(p);
-}
-__device__ __forceinline__ void mbar_init(uint64_t* bar, unsigned count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, unsigned bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)),
-               "r"(bytes)
-               : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, unsigned parity) {
-  unsigned ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-      " selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// Bounded wait for a TMA tile; gives up (status[ST_BARRIER] set) after
-// limit_ns or as soon as another wait of the launch has given up.
-__device__ __forceinline__ void mbar_wait(uint64_t* bar, unsigned parity, int* status,
-                                          long long limit_ns) {
-  if (mbar_try_wait(bar, parity)) return;
-  const long long t0 = gtimer();
-  unsigned it = 0;
-  while (!mbar_try_wait(bar, parity)) {
-    if ((++it & 63u) == 0) {
-      if (*(volatile int*)&status[ST_BARRIER] != 0) return;
-      if (gtimer() - t0 > limit_ns) {
-        atomicAdd(&status[ST_BARRIER], 1);
-        return;
-      }
-    }
-  }
-}
-// Bounded wait that reports whether the phase completed.
-__device__ __forceinline__ bool mbar_wait_ok(uint64_t* bar, unsigned parity, int* status,
-                                             long long limit_ns) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const long long t0 = gtimer();
-  unsigned it = 0;
-  while (!mbar_try_wait(bar, parity)) {
-    if ((++it & 63u) == 0) {
-      if (*(volatile int*)&status[ST_BARRIER] != 0) return false;
-      if (gtimer() - t0 > limit_ns) {
-        atomicAdd(&status[ST_BARRIER], 1);
-        return false;
-      }
-    }
-  }
-  return true;
-}
-// Before the producer leaves the kernel: every TMA copy it issued has landed
-// (q copies issued round-robin over the slots), so no copy writes into the
-// shared memory of a finished block.  Bounded by limit_ns per slot; this wait
-// ignores the status word, since the copies land whether or not a wait of the
-// launch gave up.
-template <int STAGES>
-__device__ __forceinline__ void drain_copies(uint64_t* full, unsigned q, long long limit_ns) {
-  for (unsigned s = 0; s < (unsigned)STAGES && s < q; ++s) {
-    const unsigned uses = q / STAGES + (s < q % STAGES ? 1u : 0u);
-    const unsigned parity = (uses - 1u) & 1u;
-    const long long t0 = gtimer();
-    while (!mbar_try_wait(&full[s], parity))
-      if (gtimer() - t0 > limit_ns) break;
-  }
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
 // Barrier of the TT consumer threads (named barrier 1; the producer warp does not take part).
 __device__ __forceinline__ void csync() { asm volatile("bar.sync 1, %0;" ::"n"(TT) : "memory"); }
-
-// 2-D tiled TMA load (no multicast) of one 64 x BC tile; x counts scalars
-// (re and im separately) along the rows, y counts columns.
-__device__ __forceinline__ void tma_tile(void* dst, const CUtensorMap* tm, int x, int y,
-                                         uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(dst)),
-      "l"(reinterpret_cast<uint64_t>(tm)), "r"(x), "r"(y), "r"(smem_u32(bar))
-      : "memory");
-}
 
 // Grid barrier on a monotonic arrival counter (zeroed before each launch):
 // barrier number e completes when the counter reaches e * gridDim.x (plus
@@ -231,30 +112,10 @@ struct TridArgs {
   unsigned* bar;
   int* status;
   int p, nbp, final_panel;
+  unsigned epoch0;    // barriers that earlier launches of the reduction took
   long long wait_ns;  // limit of every bounded wait
   unsigned planted;   // extra arrivals the first barrier waits for (0; a test aid)
 };
-
-__device__ __forceinline__ cplx shfl4_sum(cplx v) {
-  v.x += __shfl_xor_sync(0xffffffffu, v.x, 1);
-  v.y += __shfl_xor_sync(0xffffffffu, v.y, 1);
-  v.x += __shfl_xor_sync(0xffffffffu, v.x, 2);
-  v.y += __shfl_xor_sync(0xffffffffu, v.y, 2);
-  return v;
-}
-
-// a * conj(b)
-__device__ __forceinline__ cplx cmul_cb(cplx a, cplx b) {
-  return cmk(a.x * b.x + a.y * b.y, a.y * b.x - a.x * b.y);
-}
-
-__device__ __forceinline__ cplx warp_sum(cplx v) {
-  for (int o = 16; o > 0; o >>= 1) {
-    v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
-    v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
-  }
-  return v;
-}
 
 constexpr int JB = 8;  // column tiles whose x values are staged per round trip
 constexpr int RED_DOUBLES = NBT + 2 * NBT + 4 * NBT * NBT;  // one panel's reduction slots
@@ -329,9 +190,8 @@ __global__ void __launch_bounds__(TT + 32, 1)
   double* red_s = a.red + 3 * NBT;
   double* red_t = a.red + 3 * NBT + 2 * NBT * NBT;
   const int nch = (n + RCH - 1) / RCH;
-  // the arrival counter runs on over the panels of one reduction: the
-  // panels before column p took two barriers per column
-  unsigned epoch = 2u * (unsigned)a.p;
+  // the arrival counter runs on over the panels of one reduction
+  unsigned epoch = a.epoch0;
   unsigned gtile = 0;  // tiles consumed by this CTA (ring slot and mbarrier phase)
   if (tid == 0) {
     for (int q = 0; q < R::STAGES; ++q) {
@@ -948,47 +808,10 @@ int her2k_update(excfv_handle* h, int m2, const float2* VW, const float2* WV, lo
 int tridiag_workspace_doubles() { return 2 * RED_DOUBLES; }
 int tridiag_nb() { return NBT; }
 
-// cuTensorMapEncodeTiled through the runtime's driver entry point
-static PFN_cuTensorMapEncodeTiled_v12000 encode_tiled_fn() {
-  static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-  if (!fn) {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
-  }
-  return fn;
-}
-
-// Tensor map of the n x n matrix C (leading dimension ld) as real scalars:
-// 2n rows of re/im pairs, n columns; tiles of 64 complex rows x BC columns.
 template <typename T2>
-static int make_tile_map(CUtensorMap* tm, const T2* C, int n, long long ld) {
-  auto fn = encode_tiled_fn();
-  if (!fn) {
-    excfv_set_error("cuTensorMapEncodeTiled is not available from the driver");
-    return EXCFV_ERR_CUDA;
-  }
-  if ((reinterpret_cast<uintptr_t>(C) & 15) || ((ld * sizeof(T2)) & 15)) {
-    excfv_set_error("tridiagonal reduction: matrix base or column stride not 16-byte aligned");
-    return EXCFV_ERR_ARG;
-  }
-  const cuuint64_t dims[2] = {2ull * (cuuint64_t)n, (cuuint64_t)n};
-  const cuuint64_t strides[1] = {(cuuint64_t)ld * sizeof(T2)};
-  const cuuint32_t box[2] = {2u * RCH, (cuuint32_t)Ring<T2, 2>::BC};
-  const cuuint32_t estr[2] = {1u, 1u};
-  const CUtensorMapDataType dt =
-      (sizeof(T2) == 16) ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
-  const CUresult r = fn(tm, dt, 2, const_cast<T2*>(C), dims, strides, box, estr,
-                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) {
-    excfv_set_error("cuTensorMapEncodeTiled failed (%d) for n=%d ld=%lld", (int)r, n, ld);
-    return EXCFV_ERR_CUDA;
-  }
-  return EXCFV_OK;
-}
+int tridiag_flow_panel(excfv_handle* h, int n, int p, int nbp, int final_panel, T2* C, long long ld, T2* VW, T2* WV,
+                       int G, long long wait_ns, unsigned planted);
+int tridiag_flow_begin(excfv_handle* h, int n, int G);
 
 template <typename T2>
 int tridiag_tail_max();
@@ -1040,11 +863,17 @@ static int tridiag_reduce_t(excfv_handle* h, int n, T2* C, long long ld) {
   // each panel launch then zeroes the slots of the next
   CUDA_TRY(cudaMemsetAsync(ws.red, 0, sizeof(double) * tridiag_workspace_doubles(), s));
   CUDA_TRY(cudaMemsetAsync(ws.bar, 0, 2 * sizeof(unsigned), s));
+  int rc_flow = 0;
+  unsigned epoch0 = 0;
   const long long wait_ns = wait_limit_ns();
   const unsigned planted = take_planted_stall() ? 1u : 0u;
   // the last columns (a trailing block the cluster's shared memory holds) go
   // to the cluster kernel (tridiag_tail.cu); a planted stall keeps the panels
   const int p_tail = planted ? n : tridiag_tail_start(n, sizeof(T2) == 8);
+  // panels by the dataflow kernel where its roles suit the order and the block
+  // count (tridiag_flow.cu), else by the barrier kernel of this file
+  bool flow = ws.flow != nullptr && p_tail > 0;
+  if (flow && (rc_flow = tridiag_flow_begin(h, n, G))) return rc_flow;
   for (int p = 0; p < n - 1; p += NBT) {
     if (p == p_tail) {
       prof_begin(h, PROF_TRD_TAIL);
@@ -1055,20 +884,31 @@ static int tridiag_reduce_t(excfv_handle* h, int n, T2* C, long long ld) {
     const int nbp = min(NBT, n - 1 - p);
     const int final_panel = (p + nbp == n - 1) ? 1 : 0;
     const int pi = p / NBT;
+    if (flow) {
+      prof_begin(h, PROF_TRD_PANEL);
+      rc_flow = tridiag_flow_panel<T2>(h, n, p, nbp, final_panel, C, ld, VW, WV, G, wait_ns, (p == 0) ? planted : 0u);
+      prof_end(h, PROF_TRD_PANEL);
+      if (rc_flow < 0) return rc_flow;
+    }
+    const bool done = flow && rc_flow == 0;
     TridArgs<T2> ta;
     ta.n = n; ta.ld = ld; ta.C = C; ta.VW = VW; ta.WV = WV; ta.d = ws.d; ta.e = ws.e;
     ta.tau = ws.tau; ta.ybuf = ws.ybuf; ta.bar = ws.bar; ta.status = ws.status;
     ta.red = ws.red + (size_t)(pi & 1) * RED_DOUBLES;
     ta.red_next = ws.red + (size_t)((pi + 1) & 1) * RED_DOUBLES;
+    ta.epoch0 = epoch0;
     ta.p = p; ta.nbp = nbp; ta.final_panel = final_panel;
     ta.wait_ns = wait_ns;
     ta.planted = (p == 0) ? planted : 0u;
-    void* args[] = {&ta, &tmap};
-    prof_begin(h, PROF_TRD_PANEL);
-    CUDA_TRY(cudaLaunchCooperativeKernel((const void*)k_tridiag_panel<T2, MC>, dim3(G), dim3(TT + 32), args,
-                                         (size_t)smem, s));
-    count_launch();
-    prof_end(h, PROF_TRD_PANEL);
+    if (!done) {
+      void* args[] = {&ta, &tmap};
+      prof_begin(h, PROF_TRD_PANEL);
+      CUDA_TRY(cudaLaunchCooperativeKernel((const void*)k_tridiag_panel<T2, MC>, dim3(G), dim3(TT + 32), args,
+                                           (size_t)smem, s));
+      count_launch();
+      prof_end(h, PROF_TRD_PANEL);
+      epoch0 += 2u * (unsigned)nbp;  // two barriers per column
+    }
     if (!final_panel) {
       prof_begin(h, PROF_TRD_UPDATE);
       const int q = p + nbp;

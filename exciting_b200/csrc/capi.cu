@@ -1054,7 +1054,11 @@ long long excfv_launch_count(void) { return g_launches.load(); }
 
 int excfv_tridiag_tail_start(int n, int complex64) {
   if (n < 1) return 0;
-  return tridiag_tail_start(n, complex64 != 0);
+  int dev = 0, nsm = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    nsm = 0;
+  return tridiag_tail_start(n, complex64 != 0, nsm);
 }
 
 int excfv_set_lattice(excfv_handle* h, const double* vgc, const double* atposc) {

@@ -812,18 +812,30 @@ template <typename T2>
 int tridiag_flow_panel(excfv_handle* h, int n, int p, int nbp, int final_panel, T2* C, long long ld, T2* VW, T2* WV,
                        int G, long long wait_ns, unsigned planted);
 int tridiag_flow_begin(excfv_handle* h, int n, int G);
+bool tridiag_flow_available(int G);
 
 template <typename T2>
 int tridiag_tail_max();
 template <typename T2>
 int tridiag_tail(excfv_handle* h, int n, int c0, T2* C, long long ld);
 
-int tridiag_tail_start(int n, bool complex64) {
-  const int tail_max = complex64 ? tridiag_tail_max<float2>() : tridiag_tail_max<double2>();
+// The first panel boundary p whose trailing block goes to the cluster kernel of
+// the last columns (tridiag_tail.cu): as soon as the cluster holds the block
+// where the barrier kernel reduces the panels; where the dataflow kernel does
+// (G blocks), once the block is so small that the cluster is faster.  The
+// cluster takes 4.4 us per column below m = 200, 6.2 up to 316 and 9.2 from
+// there to 608, the dataflow panels about 6.5 with their share of the updates:
+// order 484 takes 4.76, 4.65 and 4.82 ms with the tail from 192, 320 and 448.
+constexpr int FLOW_TAIL = 320;
+static int tail_start(int n, bool complex64, int G) {
+  int tail_max = complex64 ? tridiag_tail_max<float2>() : tridiag_tail_max<double2>();
+  if (tridiag_flow_available(G)) tail_max = min(tail_max, FLOW_TAIL);
   for (int p = 0; p < n - 1; p += NBT)
     if (n - p <= tail_max) return p;
   return n > 0 ? n - 1 : 0;
 }
+
+int tridiag_tail_start(int n, bool complex64, int G) { return tail_start(n, complex64, G); }
 
 template <typename T2, int MC>
 static int tridiag_reduce_t(excfv_handle* h, int n, T2* C, long long ld) {
@@ -869,7 +881,7 @@ static int tridiag_reduce_t(excfv_handle* h, int n, T2* C, long long ld) {
   const unsigned planted = take_planted_stall() ? 1u : 0u;
   // the last columns (a trailing block the cluster's shared memory holds) go
   // to the cluster kernel (tridiag_tail.cu); a planted stall keeps the panels
-  const int p_tail = planted ? n : tridiag_tail_start(n, sizeof(T2) == 8);
+  const int p_tail = planted ? n : tail_start(n, sizeof(T2) == 8, G);
   // panels by the dataflow kernel where its roles suit the order and the block
   // count (tridiag_flow.cu), else by the barrier kernel of this file
   bool flow = ws.flow != nullptr && p_tail > 0;

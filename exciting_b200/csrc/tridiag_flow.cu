@@ -42,8 +42,9 @@
 // leave at their next block barrier, which carries the decision.
 //
 // Measured against the barrier form (panels of one solve, cluster tail apart):
-// FP64 order 715 1.36 -> 0.78 ms, 1964 17.8 -> 10.1 ms, 5028 112 -> 92 ms;
-// complex64 order 1901 13.3 -> 7.1 ms.
+// FP64 order 715 1.36 -> 0.75 ms, 1964 17.8 -> 9.7 ms, 5028 112 -> 90 ms;
+// complex64 order 1901 13.3 -> 6.8 ms.  A column takes 5.8 us at order 700, 7 at
+// 1400 and 10 at 1964, where a worker's tiles no longer all fit its ring.
 #include "tridiag_dev.cuh"
 
 namespace {
@@ -95,15 +96,19 @@ __device__ __noinline__ bool poll_expired(int* status, long long limit_ns, long 
 // the warp's carry the tag; the others read 0 (their pointers must be readable).
 // The warp stays together: lanes that left one by one ran everything up to the
 // next shuffle one after another (2 us for a dozen lanes).
+// Only the first `cnt` (the same in every lane) are loaded at all.
 template <int N>
 __device__ __forceinline__ void poll(const word* const (&ptr)[N], unsigned mask, unsigned tag, cplx (&val)[N],
-                                     Waiter& w) {
+                                     Waiter& w, int cnt = N) {
   unsigned it = 0;
   long long t0 = 0;
   for (;;) {
     unsigned long long v[N][4];
 #pragma unroll
-    for (int q = 0; q < N; ++q) ldw(ptr[q], v[q]);
+    for (int q = 0; q < N; ++q) {
+      if (q < cnt) ldw(ptr[q], v[q]);
+      else v[q][0] = v[q][1] = v[q][2] = v[q][3] = 0;
+    }
     unsigned diff = 0;  // any tag that does not match, over the wanted words
 #pragma unroll
     for (int q = 0; q < N; ++q) {
@@ -220,7 +225,7 @@ __device__ void flow_worker(const FlowArgs<T2>& a, const CUtensorMap* tmap, unsi
   __shared__ __align__(8) uint64_t s_full[FSTAGES], s_empty[FSTAGES];
   __shared__ int s_nrun, s_I[RUNMAX], s_b0[RUNMAX], s_b1[RUNMAX], s_off[RUNMAX];
   __shared__ cplx s_red[2][FT / 32][64];
-  __shared__ double s_v[2];
+  __shared__ double s_v[4];
   T2* ring = reinterpret_cast<T2*>(dsm);
   T2* sx = reinterpret_cast<T2*>(dsm + (size_t)a.stages * BYTES);   // x of the share's columns
   cplx* sxr = reinterpret_cast<cplx*>(sx + a.ecap);                  // x of the runs' rows
@@ -491,27 +496,39 @@ __device__ void flow_worker(const FlowArgs<T2>& a, const CUtensorMap* tmap, unsi
 #pragma unroll
         for (int u = 0; u < 4; ++u) s_red[k & 1][warp][rg + 16 * u] = rowp[u];
       }
+      // two runs at a time: one barrier for both
+      if (!(k & 1) && k + 1 < nrun) continue;
       bar_sync_main();
-      if (tid < 64) {
+      if (tid < 64 * (1 + (k & 1))) {
+        const int kk = (k & ~1) + (tid >> 6), r = tid & 63;
         cplx s = cmk(0.0, 0.0);
 #pragma unroll
-        for (int q = 0; q < FT / 32; ++q) s = cadd(s, s_red[k & 1][q][tid]);
-        const cplx x = sxr[k * 64 + tid];
+        for (int q = 0; q < FT / 32; ++q) s = cadd(s, s_red[kk & 1][q][r]);
+        const cplx x = sxr[kk * 64 + r];
         vav += x.x * s.x + x.y * s.y;
-        const int rel = I * 64 + tid;
-        if (rel > i && rel < nrel) stw(a.ROW + par * a.row_par + 64LL * (w + F.rank(I)) + tid, s, tag);
+        const int rel = s_I[kk] * 64 + r;
+        if (rel > i && rel < nrel) stw(a.ROW + par * a.row_par + 64LL * (w + F.rank(s_I[kk])) + r, s, tag);
       }
+      if (k + 1 < nrun) bar_sync_main();  // s_red is free again
     }
     // Re(x^H A x) of the share: its row parts count twice, the diagonal is
     // taken off by the owners
     for (int o = 16; o > 0; o >>= 1) vav += __shfl_xor_sync(0xffffffffu, vav, o);
-    if (lane == 0 && warp < 2) s_v[warp] = vav;
+    if (lane == 0 && warp < 4) s_v[warp] = vav;
     bar_sync_main();  // also: sx and sxr are free for the next column
-    if (tid == 0) stw(a.VAV + par * a.vav_par + w, cmk(2.0 * (s_v[0] + s_v[1]), 0.0), tag);
+    if (tid == 0) stw(a.VAV + par * a.vav_par + w, cmk(2.0 * (s_v[0] + s_v[1] + s_v[2] + s_v[3]), 0.0), tag);
   }
 }
 
 // ---------------------------------------------------------------------------
+// Chunk ch of owner o: block row o, then nt - 1 - o (the parts of y for a block
+// row decrease with its index, so the pairs are equally long); -1 for none.
+__device__ __forceinline__ int owner_block(int o, int ch, int nt) {
+  if (ch == 0) return o;
+  const int m = nt - 1 - o;
+  return m > o ? m : -1;
+}
+
 template <typename T2, int MC>
 struct OwnerSmem {
   T2 V[MC][NBT][RCH + 2];  // padded: a warp reads four columns of eight rows
@@ -629,8 +646,8 @@ __device__ void flow_owner(const FlowArgs<T2>& a, unsigned char* dsm, int o) {
   int rel[MC];
 #pragma unroll
   for (int ch = 0; ch < MC; ++ch) {
-    const int blk = o + ch * a.NO;
-    rel[ch] = (blk < a.nt && blk * 64 + rloc < nrel) ? blk * 64 + rloc : -1;
+    const int blk = owner_block(o, ch, a.nt);
+    rel[ch] = (blk >= 0 && blk * 64 + rloc < nrel) ? blk * 64 + rloc : -1;
     x[ch] = cn[ch] = cmk(0.0, 0.0);
     if (rel[ch] < 0) continue;
     const int r = a.p + rel[ch];
@@ -651,10 +668,10 @@ __device__ void flow_owner(const FlowArgs<T2>& a, unsigned char* dsm, int o) {
   long long rofs[MC];
 #pragma unroll
   for (int ch = 0; ch < MC; ++ch) {
-    const int I = o + ch * a.NO;  // the chunk's block row
+    const int I = owner_block(o, ch, a.nt);
     nrow[ch] = ncon[ch] = 0;
     rofs[ch] = 0;
-    if (I >= a.nt) continue;
+    if (I < 0) continue;
     const long long rs = F.row_begin(I);
     const int w0 = worker_of(rs, F.U, a.NW), w1 = worker_of(rs + (long long)(I + 1) * BPT - 1, F.U, a.NW);
     nrow[ch] = w1 - w0 + 1;
@@ -741,10 +758,10 @@ __device__ void flow_owner(const FlowArgs<T2>& a, unsigned char* dsm, int o) {
       s_tv[tid] = cadd(cmul(scale, s_T[tid]), cconj(wc));
     }
     if (bar_owner(wt.bad)) return;
-    cplx q[MC], u[MC], y[MC];
+    cplx q[MC], u[MC];
 #pragma unroll
     for (int ch = 0; ch < MC; ++ch) {
-      q[ch] = u[ch] = y[ch] = cmk(0.0, 0.0);
+      q[ch] = u[ch] = cmk(0.0, 0.0);
       const bool act = rel[ch] >= i + 1;
       if (act) {
         cplx q2 = cmk(0.0, 0.0), u2 = cmk(0.0, 0.0);
@@ -767,11 +784,13 @@ __device__ void flow_owner(const FlowArgs<T2>& a, unsigned char* dsm, int o) {
       q[ch] = shfl4_sum(q[ch]);
       u[ch] = shfl4_sum(u[ch]);
     }
+    cplx y[MC];
     // y = C22 x: row parts of the workers that share the block row, then the
     // column parts of this and all later block rows
 #pragma unroll
     for (int ch = 0; ch < MC; ++ch) {
-      const int I = o + ch * a.NO, r0 = I * 64;
+      y[ch] = cmk(0.0, 0.0);
+      const int I = max(owner_block(o, ch, a.nt), 0), r0 = I * 64;
       // rows past the matrix or above the column poll a row of the block that is sent
       const bool act = rel[ch] >= i + 1;
       const int rmin = max(i + 1 - r0, 0), rmax = min(63, nrel - 1 - r0);
@@ -796,7 +815,7 @@ __device__ void flow_owner(const FlowArgs<T2>& a, unsigned char* dsm, int o) {
           ptr[h] = (kk < nrow[ch] ? rb + 64 * kk : cb + col_at(I + kk - nrow[ch], 0)) + rr;
           if (act && k + 4 * h < ncon[ch]) mask |= 1u << h;
         }
-        poll(ptr, mask, tag, v, wt);
+        poll(ptr, mask, tag, v, wt, (ncon[ch] - (k - rsub) + 3) >> 2);
         y[ch] = cadd(y[ch], cadd(cadd(cadd(v[0], v[1]), cadd(v[2], v[3])), cadd(cadd(v[4], v[5]), cadd(v[6], v[7]))));
       }
       y[ch] = shfl4_sum(y[ch]);
@@ -912,6 +931,9 @@ int flow_panel(excfv_handle* h, const CUtensorMap& tmap, FlowArgs<T2> a, int G, 
 
 // Bytes of the words for orders up to n.
 size_t tridiag_flow_bytes(int n, int nsm) { return (size_t)FlowLayout(n, nsm).total * sizeof(word); }
+
+// Whether G blocks are enough for the roles at all (of the smaller trailing blocks).
+bool tridiag_flow_available(int G) { return G - 16 >= NK; }
 
 // Zeroes the words of the reduction that begins (tags of an earlier one must
 // not be taken).

@@ -519,9 +519,10 @@ int excfv_profile_read(excfv_handle* h, double* ms, long long* count, int nclass
 long long excfv_launch_count(void);
 
 /* The first column of the tridiagonal reduction of an n x n matrix that its
- * cluster kernel reduces (the trailing block from there on fits in the
- * cluster's shared memory; the panel kernel takes the columns before it);
- * n - 1 when no column goes there.  complex64 != 0 for the precision form's
+ * cluster kernel reduces on the current device (the trailing block from there
+ * on fits in the cluster's shared memory and is small enough for it to be the
+ * faster one; the panel kernels take the columns before it); n - 1 when no
+ * column goes there.  complex64 != 0 for the precision form's
  * complex64 storage, 0 for FP64. */
 int excfv_tridiag_tail_start(int n, int complex64);
 

@@ -113,7 +113,7 @@ void excfv_set_error(const char* fmt, ...) {
 
 void free_static(DevStatic& st) {
   dfree(st.idxis); dfree(st.rmt); dfree(st.apword); dfree(st.flist); dfree(st.fofl);
-  dfree(st.lo_atom); dfree(st.lo_local); dfree(st.lo_lm); dfree(st.lo_ilo);
+  dfree(st.lo_atom); dfree(st.lo_local); dfree(st.lo_first); dfree(st.lo_lm); dfree(st.lo_ilo);
   dfree(st.aa); dfree(st.loa); dfree(st.lolo); dfree(st.oalo); dfree(st.ololo); dfree(st.h1aa);
   dfree(st.ivg); dfree(st.ivgig); dfree(st.veffig); dfree(st.xig); dfree(st.cfunig);
   dfree(st.m2effig); dfree(st.zdinv);
@@ -301,6 +301,9 @@ int stage_set_static(excfv_handle* h, const excfv_static* s) {
   if ((rc = upload(&st.fofl, fofl.data(), fofl.size()))) return rc;
   if ((rc = upload(&st.lo_atom, lo_atom.data(), lo_atom.size()))) return rc;
   if ((rc = upload(&st.lo_local, lo_local.data(), lo_local.size()))) return rc;
+  std::vector<int> lo_first(na, -1);
+  for (int a = 0; a < na && a < (int)st.h_lo_first.size(); ++a) lo_first[a] = st.h_lo_first[a];
+  if ((rc = upload(&st.lo_first, lo_first.data(), lo_first.size()))) return rc;
   if ((rc = upload(&st.lo_lm, lo_lm.data(), lo_lm.size()))) return rc;
   if ((rc = upload(&st.lo_ilo, lo_ilo.data(), lo_ilo.size()))) return rc;
   if ((rc = upload(&st.aa, s->aa, (size_t)st.maxaa * st.maxaa * na))) return rc;

@@ -32,6 +32,7 @@ struct DevStatic {
   int* fofl = nullptr;      // (lmmaxapw*apwordmax, nspecies) inverse of flist, -1 unused
   int* lo_atom = nullptr;   // (nlotot) atom of each LO function
   int* lo_local = nullptr;  // (nlotot) index inside the atom's LO block
+  int* lo_first = nullptr;  // (natmtot) first global LO index, -1 none
   int* lo_lm = nullptr;     // (maxnlo, natmtot) lm of LO function j of the atom
   int* lo_ilo = nullptr;    // (maxnlo, natmtot) ilo of LO function j
   cplx* aa = nullptr;       // (maxaa, maxaa, natmtot)

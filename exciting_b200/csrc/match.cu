@@ -64,33 +64,44 @@ __global__ void k_zdinv(int natmtot, int lmaxapw, int apwordmax, int np, const i
       out[i + apwordmax * j] = (i < nap && j < nap) ? inv[i][j] : 0.0;
 }
 
-// One thread per G+k: Y_lm (ylm[ig*lmmax + lm]) and, per species, the Bessel
-// derivatives |G+k|^j j_l^{(j)}(|G+k| R), djl[((is*ngkmax + ig)*(lmax+1) + l)*apwordmax + j].
+// Y_lm (ylm[ig*lmmax + lm]) and, per species, the Bessel derivatives
+// |G+k|^j j_l^{(j)}(|G+k| R), djl[((is*ngkmax + ig)*(lmax+1) + l)*apwordmax + j].
+// One thread per G+k and task (blockIdx.y): one m of Y_lm, or one species' order
+// j.  The recurrences are serial chains, so the time is that of the longest: with
+// all tasks of a G+k in one thread it was 47 us for any number of G+k below
+// 19000, as tasks it is 19.5 us.
 __global__ void k_ylm_bessel(int ngp, int ngkmax, int lmax, int apwordmax, int nspecies,
                              const int* apword, const double* rmt, const double* gpc,
                              const double* tpgpc, cplx* ylm, double* djl) {
   const int ig = blockIdx.x * blockDim.x + threadIdx.x;
   if (ig >= ngp) return;
   const int lmmax = (lmax + 1) * (lmax + 1);
-  sf_ylm(lmax, tpgpc[2 * ig], tpgpc[2 * ig + 1], ylm + (size_t)ig * lmmax, 1);
+  if ((int)blockIdx.y <= lmax) {
+    const int m = blockIdx.y;
+    const double theta = tpgpc[2 * ig], phi = tpgpc[2 * ig + 1];
+    const double ct = cos(theta), st = sin(theta);
+    const cplx rot = cmk(cos(phi), sin(phi));
+    cplx eim = cmk(1.0, 0.0);
+    double pmm = 0.28209479177387814347;
+    for (int q = 1; q <= m; ++q) sf_ylm_step(q, st, rot, pmm, eim);
+    sf_ylm_m(lmax, m, ct, pmm, eim, ylm + (size_t)ig * lmmax, 1);
+    return;
+  }
+  const int b = blockIdx.y - (lmax + 1), is = b / apwordmax, j = b % apwordmax;
   const double g = gpc[ig];
   double buf[LMAX_CAP + 1];
-  for (int is = 0; is < nspecies; ++is) {
-    int omax = 0;
-    for (int l = 0; l <= lmax; ++l) omax = max(omax, apword[l + (lmax + 1) * is]);
-    const double x = g * rmt[is];
+  int omax = 0;
+  for (int l = 0; l <= lmax; ++l) omax = max(omax, apword[l + (lmax + 1) * is]);
+  double* dj = djl + ((size_t)is * ngkmax + ig) * (lmax + 1) * apwordmax + j;
+  if (j < omax) {
     double sc = 1.0;
-    for (int j = 0; j < omax; ++j) {
-      sf_sbessel_deriv(j, lmax, x, buf);
-      for (int l = 0; l <= lmax; ++l)
-        djl[(((size_t)is * ngkmax + ig) * (lmax + 1) + l) * apwordmax + j] = sc * buf[l];
-      sc *= g;
-    }
+    for (int q = 0; q < j; ++q) sc *= g;
+    sf_sbessel_deriv(j, lmax, g * rmt[is], buf);
+    for (int l = 0; l <= lmax; ++l) dj[l * apwordmax] = sc * buf[l];
+  } else {
     // orders past this species' largest apword are multiplied by zero later;
     // store zeros so that no uninitialised value (possibly a NaN) takes part
-    for (int j = omax; j < apwordmax; ++j)
-      for (int l = 0; l <= lmax; ++l)
-        djl[(((size_t)is * ngkmax + ig) * (lmax + 1) + l) * apwordmax + j] = 0.0;
+    for (int l = 0; l <= lmax; ++l) dj[l * apwordmax] = 0.0;
   }
 }
 
@@ -200,7 +211,8 @@ int stage_match(excfv_handle* h, int ngp, int ngkmax, cplx* apwalm_ref) {
   if (st.lmaxapw > LMAX_CAP) return EXCFV_ERR_UNSUPPORTED;
   const double fpso = 4.0 * M_PI / sqrt(st.omega);
   prof_begin(h, PROF_MATCH);
-  k_ylm_bessel<<<(ngp + 127) / 128, 128, 0, s>>>(ngp, ws.ngkmax, st.lmaxapw, st.apwordmax,
+  const dim3 tasks((ngp + 63) / 64, st.lmaxapw + 1 + st.nspecies * st.apwordmax);
+  k_ylm_bessel<<<tasks, 64, 0, s>>>(ngp, ws.ngkmax, st.lmaxapw, st.apwordmax,
                                                  st.nspecies, st.apword, st.rmt, ws.gpc,
                                                  ws.tpgpc, ws.ylm, ws.djl); count_launch();
   CUDA_TRY(cudaGetLastError());
@@ -312,7 +324,8 @@ extern "C" int excfv_match_noalloc(excfv_handle* h, int32_t ngp, int32_t ngkmax,
     double* djl = reinterpret_cast<double*>(base + djl_off);
     const double fpso = 4.0 * M_PI / sqrt(st.omega);
     cudaStream_t s = h->stream;
-    k_ylm_bessel<<<(ngp + 127) / 128, 128, 0, s>>>(ngp, ngkmax, st.lmaxapw, st.apwordmax, st.nspecies,
+    const dim3 tasks((ngp + 63) / 64, st.lmaxapw + 1 + st.nspecies * st.apwordmax);
+    k_ylm_bessel<<<tasks, 64, 0, s>>>(ngp, ngkmax, st.lmaxapw, st.apwordmax, st.nspecies,
                                                    st.apword, st.rmt, gpc, tpgpc, ylm, djl);
     count_launch();
     const long long tr = (long long)ngkmax * st.apwordmax * st.lmmaxapw * st.natmtot;

@@ -17,53 +17,93 @@
 
 namespace {
 
-// LO band: columns N..n-1, rows 0..j (assigned, not accumulated).
-// H(G, lo) = conj(loa * apwi)^T (hamiltonsetup.f90:131-149),
-// O(G, lo_m) = conj(A(G, io, lm) (oalo + h1loa)) (overlapsetup.f90:119-131),
-// H(lo, lo') = lolo (:154-161), O(lo_m, lo'_m) = ololo + h1lolo (:136-148).
-__global__ void k_lo_band(int N, int n, int natmtot, int maxaa, int maxnlo, int nlomax,
-                          int apwordmax, const int* idxis, const int* lo_atom, const int* lo_local,
-                          const int* lo_lm, const int* lo_ilo, const int* fofl, int lmmax,
-                          const cplx* Apk, const cplx* loa, const cplx* lolo, const double* oalo,
-                          const double* ololo, cplx* H, cplx* O, long long ld) {
-  const int j = N + blockIdx.y;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= n || i > j) return;
-  const int jl = j - N;
-  const int a = lo_atom[jl], jj = lo_local[jl];
-  const int lmj = lo_lm[jj + maxnlo * a], iloj = lo_ilo[jj + maxnlo * a];
-  cplx hv = cmk(0.0, 0.0), ov = cmk(0.0, 0.0);
+// LO band: columns N..n-1, rows 0..j (assigned, not accumulated), in two kernels.
+// G+k rows: H(G, lo) = conj(loa * apwi)^T (hamiltonsetup.f90:131-149),
+// O(G, lo_m) = conj(A(G, io, lm) (oalo + h1loa)) (overlapsetup.f90:119-131).
+// A warp takes one G+k vector of one atom: its packed coefficients are read once,
+// coalesced, for up to LOJ of the atom's functions at a time, whose loa rows are
+// staged in shared memory.  8 atoms with 8 functions each: N = 1900 131 -> 73 us,
+// 2 atoms, N = 300 31 -> 11 us against a thread per element, which read the
+// coefficients uncoalesced once per function.
+constexpr int LOJ = 8;    // functions per pass
+constexpr int LOW = 8;    // warps (G+k vectors) per CTA
+__global__ void __launch_bounds__(32 * LOW) k_lo_gk(int N, int natmtot, int maxaa, int maxnlo, int nlomax,
+                                                    int apwordmax, const int* idxis, const int* lo_first,
+                                                    const int* lo_lm, const int* lo_ilo, const int* fofl, int lmmax,
+                                                    const cplx* __restrict__ Apk, const cplx* __restrict__ loa,
+                                                    const double* oalo, cplx* H, cplx* O, long long ld, int staged) {
+  extern __shared__ __align__(16) unsigned char lsm[];
+  cplx* sl = reinterpret_cast<cplx*>(lsm);  // [LOJ][maxaa]
+  const int a = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (lo_first[a] < 0) return;
+  const int is = idxis[a];
   const long long AM = (long long)natmtot * maxaa;
-  if (i < N) {
-    const cplx* ac = Apk + (long long)a * maxaa + AM * i;
-    const cplx* lr = loa + jj + (long long)maxnlo * maxaa * a;
-    // (loa * apwi)(jj, i) = sum_f loa(jj, f) A(i, f); we need its conjugate
-    double re = 0.0, im = 0.0;
-    for (int f = 0; f < maxaa; ++f) {
-      const cplx x = lr[(long long)maxnlo * f];
-      const cplx y = ac[f];
-      re += x.x * y.x - x.y * y.y;
-      im += x.x * y.y + x.y * y.x;
+  for (int q0 = 0; q0 < maxnlo; q0 += LOJ) {
+    __syncthreads();
+    for (int t = threadIdx.x; staged && t < LOJ * maxaa; t += 32 * LOW) {
+      const int q = q0 + t % LOJ, f = t / LOJ;
+      sl[t % LOJ * maxaa + f] = (q < maxnlo) ? loa[q + (long long)maxnlo * (f + (long long)maxaa * a)] : cmk(0.0, 0.0);
     }
-    hv = cmk(re, -im);
-    const int is = idxis[a];
-    for (int io = 0; io < apwordmax; ++io) {
-      const int f = fofl[(lmj * apwordmax + io) + lmmax * apwordmax * is];
-      if (f < 0) continue;
-      const cplx y = ac[f];
-      const double c = oalo[io + apwordmax * (iloj + (long long)nlomax * a)];
-      ov.x += c * y.x;
-      ov.y -= c * y.y;
-    }
-  } else {
-    const int il = i - N;
-    if (lo_atom[il] == a) {
-      const int ii = lo_local[il];
-      hv = lolo[ii + maxnlo * (jj + (long long)maxnlo * a)];
-      if (lo_lm[ii + maxnlo * a] == lmj) {
-        const int iloi = lo_ilo[ii + maxnlo * a];
-        ov = cmk(ololo[iloi + nlomax * (iloj + (long long)nlomax * a)], 0.0);
+    __syncthreads();
+    for (int i = blockIdx.x * LOW + warp; i < N; i += gridDim.x * LOW) {
+      const cplx* ac = Apk + (long long)a * maxaa + AM * i;
+      cplx v[LOJ];
+#pragma unroll
+      for (int q = 0; q < LOJ; ++q) v[q] = cmk(0.0, 0.0);
+      for (int f = lane; f < maxaa; f += 32) {
+        const cplx y = ac[f];
+#pragma unroll
+        for (int q = 0; q < LOJ; ++q) {
+          // (a very large basis does not fit the shared memory)
+          const cplx l = staged ? sl[q * maxaa + f]
+                                : loa[min(q0 + q, maxnlo - 1) + (long long)maxnlo * (f + (long long)maxaa * a)];
+          v[q] = cadd(v[q], cmul(l, y));
+        }
       }
+#pragma unroll
+      for (int q = 0; q < LOJ; ++q)
+        for (int o = 16; o > 0; o >>= 1) {
+          v[q].x += __shfl_xor_sync(0xffffffffu, v[q].x, o);
+          v[q].y += __shfl_xor_sync(0xffffffffu, v[q].y, o);
+        }
+#pragma unroll
+      for (int q = 0; q < LOJ; ++q) {
+        if (lane != q || q0 + q >= maxnlo) continue;
+        const int jj = q0 + q, lm = lo_lm[jj + maxnlo * a];
+        if (lm < 0) continue;  // the atom has fewer functions
+        cplx ov = cmk(0.0, 0.0);
+        for (int io = 0; io < apwordmax; ++io) {
+          const int f = fofl[(lm * apwordmax + io) + lmmax * apwordmax * is];
+          if (f < 0) continue;
+          const cplx y = ac[f];
+          const double c = oalo[io + apwordmax * (lo_ilo[jj + maxnlo * a] + (long long)nlomax * a)];
+          ov.x += c * y.x;
+          ov.y -= c * y.y;
+        }
+        const long long at = i + ld * (N + lo_first[a] + jj);
+        H[at] = cmk(v[q].x, -v[q].y);
+        O[at] = ov;
+      }
+    }
+  }
+}
+
+// LO rows: H(lo, lo') = lolo (:154-161), O(lo_m, lo'_m) = ololo + h1lolo (:136-148)
+__global__ void k_lo_lo(int N, int n, int maxnlo, int nlomax, const int* lo_atom, const int* lo_local,
+                        const int* lo_lm, const int* lo_ilo, const cplx* lolo, const double* ololo, cplx* H, cplx* O,
+                        long long ld) {
+  const int j = N + blockIdx.y;
+  const int i = N + blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= n || i > j) return;
+  const int jl = j - N, il = i - N;
+  const int a = lo_atom[jl], jj = lo_local[jl];
+  cplx hv = cmk(0.0, 0.0), ov = cmk(0.0, 0.0);
+  if (lo_atom[il] == a) {
+    const int ii = lo_local[il];
+    hv = lolo[ii + maxnlo * (jj + (long long)maxnlo * a)];
+    if (lo_lm[ii + maxnlo * a] == lo_lm[jj + maxnlo * a]) {
+      const int iloi = lo_ilo[ii + maxnlo * a], iloj = lo_ilo[jj + maxnlo * a];
+      ov = cmk(ololo[iloi + nlomax * (iloj + (long long)nlomax * a)], 0.0);
     }
   }
   H[i + ld * j] = hv;
@@ -284,11 +324,17 @@ int stage_setup(excfv_handle* h, int nmatp, int ngp, bool mirror_o) {
   prof_begin(h, PROF_SETUP_OTHER);
   // local-orbital band (columns N..n-1)
   if (n > N) {
-    dim3 grid((n + 127) / 128, n - N);
-    k_lo_band<<<grid, 128, 0, s>>>(N, n, st.natmtot, st.maxaa, st.maxnlo, st.nlomax, st.apwordmax,
-                                   st.idxis, st.lo_atom, st.lo_local, st.lo_lm, st.lo_ilo,
-                                   st.fofl, st.lmmaxapw, ws.Apk, st.loa, st.lolo, st.oalo,
-                                   st.ololo, ws.H, ws.O, ld); count_launch();
+    const bool staged = sizeof(cplx) * LOJ * st.maxaa <= 160 * 1024;
+    const int smem = staged ? (int)(sizeof(cplx) * LOJ * st.maxaa) : 0;
+    CUDA_TRY(cudaFuncSetAttribute(k_lo_gk, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    const int gx = min((N + LOW - 1) / LOW, max(1, 8 * h->nsm / st.natmtot));
+    k_lo_gk<<<dim3(gx, st.natmtot), 32 * LOW, smem, s>>>(N, st.natmtot, st.maxaa, st.maxnlo, st.nlomax, st.apwordmax,
+                                                         st.idxis, st.lo_first, st.lo_lm, st.lo_ilo, st.fofl,
+                                                         st.lmmaxapw, ws.Apk, st.loa, st.oalo, ws.H, ws.O, ld, staged);
+    count_launch();
+    k_lo_lo<<<dim3((n - N + 127) / 128, n - N), 128, 0, s>>>(N, n, st.maxnlo, st.nlomax, st.lo_atom, st.lo_local,
+                                                             st.lo_lm, st.lo_ilo, st.lolo, st.ololo, ws.H, ws.O, ld);
+    count_launch();
     CUDA_TRY(cudaGetLastError());
   }
   // interstitial

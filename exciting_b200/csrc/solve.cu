@@ -39,8 +39,13 @@ constexpr int LT = 256;
 // Triangular factor of the block reflector H_p ... H_{p+nb-1} = I - V T V^H
 // (forward, columnwise: T(i,i) = tau_i, T(0:i,i) = -tau_i T(0:i,0:i) G(0:i,i)
 // with G = V^H V), for the NBQ-wide diagonal sub-blocks of the NBW blocks.
-// One CTA per sub-block; G and T live in shared memory, four threads share
-// each row of the triangular product.
+// One CTA per sub-block, G and T in shared memory: a warp per 16-wide leaf runs
+// the recurrence (15 steps without block barriers), then pairs are merged twice,
+//   T([V1 V2]) = [[T1, -T1 (G12 T2)], [0, T2]],
+// the products G12 T2 in G's unused lower blocks.  26 us; the recurrence over
+// all 64 columns with two block barriers each took 48 us.
+constexpr int LEAF = 16;
+
 __global__ void __launch_bounds__(LT) k_larft(int n, const cplx* Gbig, const cplx* tau, cplx* Tbig) {
   extern __shared__ __align__(16) unsigned char dsm[];
   cplx (*G)[NBQ + 1] = reinterpret_cast<cplx (*)[NBQ + 1]>(dsm);
@@ -49,7 +54,7 @@ __global__ void __launch_bounds__(LT) k_larft(int n, const cplx* Gbig, const cpl
   const int p = blk * NBQ;
   const int nb = min(NBQ, n - 1 - p);
   if (nb <= 0) return;
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const cplx* Gb = Gbig + (size_t)p * (NBW + 1);
   for (int t = tid; t < NBQ * NBQ; t += LT) {
     const int r = t % NBQ, c = t / NBQ;
@@ -57,21 +62,36 @@ __global__ void __launch_bounds__(LT) k_larft(int n, const cplx* Gbig, const cpl
     T[r][c] = cmk(0.0, 0.0);
   }
   __syncthreads();
-  if (tid == 0) T[0][0] = tau[p];
+  if (warp < NBQ / LEAF) {
+    const int o = warp * LEAF, row = o + (lane >> 1), sub = lane & 1;
+    for (int i = o; i < min(o + LEAF, nb); ++i) {
+      const cplx ti = tau[p + i];
+      cplx val = cmk(0.0, 0.0);
+      if (row < i)
+        for (int q = row + sub; q < i; q += 2) val = cadd(val, cmul(T[row][q], G[q][i]));
+      val.x += __shfl_xor_sync(0xffffffffu, val.x, 1);
+      val.y += __shfl_xor_sync(0xffffffffu, val.y, 1);
+      if (row < i && sub == 0) T[row][i] = cmul(cmk(-ti.x, -ti.y), val);
+      if (row == i && sub == 0) T[i][i] = ti;
+      __syncwarp();
+    }
+  }
   __syncthreads();
-  const int row = tid >> 2, sub = tid & 3;
-  for (int i = 1; i < nb; ++i) {
-    const cplx ti = tau[p + i];
-    cplx val = cmk(0.0, 0.0);
-    if (row < i)
-      for (int q = row + sub; q < i; q += 4) val = cadd(val, cmul(T[row][q], G[q][i]));
-    val.x += __shfl_xor_sync(0xffffffffu, val.x, 1);
-    val.y += __shfl_xor_sync(0xffffffffu, val.y, 1);
-    val.x += __shfl_xor_sync(0xffffffffu, val.x, 2);
-    val.y += __shfl_xor_sync(0xffffffffu, val.y, 2);
+  for (int bs = LEAF; bs < NBQ; bs *= 2) {
+    const int npair = NBQ / (2 * bs), tot = npair * bs * bs;
+    for (int t = tid; t < tot; t += LT) {  // X = G12 T2
+      const int o = t / (bs * bs) * 2 * bs, r = t % bs, c = t % (bs * bs) / bs;
+      cplx v = cmk(0.0, 0.0);
+      for (int q = 0; q <= c; ++q) v = cadd(v, cmul(G[o + r][o + bs + q], T[o + bs + q][o + bs + c]));
+      G[o + bs + r][o + c] = v;
+    }
     __syncthreads();
-    if (row < i && sub == 0) T[row][i] = cmul(cmk(-ti.x, -ti.y), val);
-    if (tid == 0) T[i][i] = ti;
+    for (int t = tid; t < tot; t += LT) {  // T12 = -T1 X
+      const int o = t / (bs * bs) * 2 * bs, r = t % bs, c = t % (bs * bs) / bs;
+      cplx v = cmk(0.0, 0.0);
+      for (int q = r; q < bs; ++q) v = cadd(v, cmul(T[o + r][o + q], G[o + bs + q][o + c]));
+      T[o + r][o + bs + c] = cmk(-v.x, -v.y);
+    }
     __syncthreads();
   }
   cplx* out = Tbig + (size_t)p * (NBW + 1);
@@ -546,13 +566,13 @@ int stage_solve_back(excfv_handle* h, int n, int k, double evaltol, double* d_ev
                      long long ldevec) {
   if (h->prec == EXCFV_PREC_MIXED && n > 64)
     return stage_solve_mixed(h, n, k, evaltol, d_eval, d_evec, ldevec);
-  return solve_back_fp64(h, n, k, evaltol, d_eval, d_evec, ldevec);
+  return solve_back_fp64(h, n, k, evaltol, d_eval, d_evec, ldevec, false);
 }
 
 // From C (ws.H) and Ui onwards: tridiagonal reduction, eigenpairs of T,
 // back-transforms.
 static int solve_back_fp64(excfv_handle* h, int n, int k, double evaltol, double* d_eval, cplx* d_evec,
-                           long long ldevec) {
+                           long long ldevec, bool standard) {
   Workspace& ws = h->ws;
   cudaStream_t s = h->stream;
   const long long ld = n;

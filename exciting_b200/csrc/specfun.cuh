@@ -23,40 +23,45 @@ constexpr int SPECFUN_MAXD = 6;    // highest radial derivative
 //                a(l,m) = sqrt((4l^2 - 1) / (l^2 - m^2)),
 // Y_lm = Pb(l, m) e^{i m phi} with e^{i m phi} advanced by one complex
 // rotation per m, and Y_l,-m = (-1)^m conj(Y_lm).
+// sf_ylm_m does one m (and -m) of it, sf_ylm all.
+EXCFV_HD void sf_ylm_m(int lmax, int m, double ct, double pmm, cplx eim, cplx* ylm, int stride) {
+  double p2 = 0.0, p1 = pmm;       // Pb(l-2, m), Pb(l-1, m) entering l = m + 1
+  for (int l = m; l <= lmax; ++l) {
+    double p;
+    if (l == m) {
+      p = pmm;
+    } else if (l == m + 1) {
+      p = sqrt(2.0 * m + 3.0) * ct * pmm;
+      p2 = pmm;
+      p1 = p;
+    } else {
+      const double a = sqrt((4.0 * l * l - 1.0) / ((double)l * l - (double)m * m));
+      const double ap = sqrt((4.0 * (l - 1) * (l - 1) - 1.0) / ((double)(l - 1) * (l - 1) - (double)m * m));
+      p = a * (ct * p1 - p2 / ap);
+      p2 = p1;
+      p1 = p;
+    }
+    const int c = l * (l + 1);
+    const cplx y = cmk(p * eim.x, p * eim.y);
+    ylm[(c + m) * stride] = y;
+    if (m > 0) {
+      const double sg = (m & 1) ? -1.0 : 1.0;
+      ylm[(c - m) * stride] = cmk(sg * y.x, -sg * y.y);
+    }
+  }
+}
+EXCFV_HD void sf_ylm_step(int m, double st, cplx rot, double& pmm, cplx& eim) {  // from m - 1 to m
+  pmm *= -sqrt((2.0 * m + 1.0) / (2.0 * m)) * st;
+  eim = cmul(eim, rot);
+}
 EXCFV_HD void sf_ylm(int lmax, double theta, double phi, cplx* ylm, int stride) {
   const double ct = cos(theta), st = sin(theta);
   const cplx rot = cmk(cos(phi), sin(phi));
   cplx eim = cmk(1.0, 0.0);           // e^{i m phi}
   double pmm = 0.28209479177387814347;  // Pb(m, m); 1 / sqrt(4 pi) at m = 0
   for (int m = 0; m <= lmax; ++m) {
-    if (m > 0) {
-      pmm *= -sqrt((2.0 * m + 1.0) / (2.0 * m)) * st;
-      eim = cmul(eim, rot);
-    }
-    double p2 = 0.0, p1 = pmm;       // Pb(l-2, m), Pb(l-1, m) entering l = m + 1
-    for (int l = m; l <= lmax; ++l) {
-      double p;
-      if (l == m) {
-        p = pmm;
-      } else if (l == m + 1) {
-        p = sqrt(2.0 * m + 3.0) * ct * pmm;
-        p2 = pmm;
-        p1 = p;
-      } else {
-        const double a = sqrt((4.0 * l * l - 1.0) / ((double)l * l - (double)m * m));
-        const double ap = sqrt((4.0 * (l - 1) * (l - 1) - 1.0) / ((double)(l - 1) * (l - 1) - (double)m * m));
-        p = a * (ct * p1 - p2 / ap);
-        p2 = p1;
-        p1 = p;
-      }
-      const int c = l * (l + 1);
-      const cplx y = cmk(p * eim.x, p * eim.y);
-      ylm[(c + m) * stride] = y;
-      if (m > 0) {
-        const double sg = (m & 1) ? -1.0 : 1.0;
-        ylm[(c - m) * stride] = cmk(sg * y.x, -sg * y.y);
-      }
-    }
+    if (m > 0) sf_ylm_step(m, st, rot, pmm, eim);
+    sf_ylm_m(lmax, m, ct, pmm, eim, ylm, stride);
   }
 }
 

@@ -1,8 +1,8 @@
 // Eigenpairs of the real symmetric tridiagonal T = tridiag(e, d, e).
 //
-// Eigenvalues (DSTEBZ, external/LAPACK/zheevx.f:490, range 'I'): one warp
-// per requested eigenvalue index, multisection on the Sturm count (32
-// points per step, the interval shrinks 33x per step) from the Gershgorin
+// Eigenvalues (DSTEBZ, external/LAPACK/zheevx.f:490, range 'I'): one CTA of T
+// threads per requested eigenvalue index, multisection on the Sturm count (T
+// points per step, the interval shrinks T + 1 times) from the Gershgorin
 // interval; stop when the width is below max(abstol, pivmin,
 // 2 ulp max(|lo|,|hi|)) exactly as DSTEBZ's bisection test.
 //
@@ -89,11 +89,11 @@ __global__ void k_tridiag_prep(int n, const double* d, const double* e, double* 
   }
 }
 
+// One CTA per eigenvalue index; all its threads are the points of a step.
 __global__ void k_stebz(int n, const double* d, const double* e2, const double* scal, int k,
                         double abstol, double* w, int* status) {
-  const int j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (j >= k) return;
+  __shared__ int s_first[2][32];
+  const int j = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, T = blockDim.x;
   const double pivmin = scal[2];
   const double ulp = 2.220446049250313e-16;
   const double atol = abstol > 0.0 ? abstol : ulp * scal[3];
@@ -103,23 +103,20 @@ __global__ void k_stebz(int n, const double* d, const double* e2, const double* 
     const double width = hi - lo;
     const double tol = fmax(fmax(atol, pivmin), 2.0 * ulp * fmax(fabs(lo), fabs(hi)));
     if (width <= tol) { conv = true; break; }
-    const double step = width / 33.0;
-    double x = lo + (lane + 1) * step;
-    if (x >= hi) x = hi;
-    const int cnt = sturm_count(n, d, e2, x, pivmin);
+    const double step = width / (T + 1);
+    const int cnt = sturm_count(n, d, e2, fmin(lo + (tid + 1) * step, hi), pivmin);
+    // the first point with at least j + 1 eigenvalues below it (T: none)
     const unsigned ball = __ballot_sync(0xffffffffu, cnt >= j + 1);
-    if (ball == 0u) {
-      lo = __shfl_sync(0xffffffffu, x, 31);
-    } else {
-      const int f = __ffs(ball) - 1;
-      const double xf = __shfl_sync(0xffffffffu, x, f);
-      const double xp = __shfl_sync(0xffffffffu, x, f > 0 ? f - 1 : 0);
-      hi = xf;
-      if (f > 0) lo = xp;
-    }
+    if (lane == 0) s_first[it & 1][warp] = ball ? 32 * warp + __ffs(ball) - 1 : T;
+    __syncthreads();
+    int f = T;
+    for (int q = 0; q < T / 32; ++q) f = min(f, s_first[it & 1][q]);
+    const double l0 = lo;
+    if (f > 0) lo = fmin(l0 + f * step, hi);
+    if (f < T) hi = fmin(l0 + (f + 1) * step, hi);
     if (!(hi > lo)) { conv = true; break; }
   }
-  if (lane == 0) {
+  if (tid == 0) {
     w[j] = 0.5 * (lo + hi);
     if (!conv) atomicAdd(&status[ST_STEBZ], 1);
   }
@@ -430,7 +427,14 @@ int tridiag_eig(excfv_handle* h, int n, int k, double abstol, const double* d, c
   double* Yi = um + (size_t)n * k;
   k_tridiag_prep<<<1, 256, 0, s>>>(n, d, e, e2, scal); count_launch();
   CUDA_TRY(cudaGetLastError());
-  k_stebz<<<(k * 32 + 127) / 128, 128, 0, s>>>(n, d, e2, scal, k, abstol, w, h->ws.status); count_launch();
+  // A step costs a Sturm chain of n dependent steps (82 clocks each) however many
+  // points it has, until the reciprocals fill their unit at about 8 warps per SM
+  // of the handle's budget: as many points as that allows (k = 20: 256 points and
+  // 7 steps instead of 32 and 10; 1024 points took 215 us where 32 took 160).
+  const int sms = (h->grid_ctas > 0) ? h->grid_ctas : h->nsm;
+  int T = 32;
+  while (T < 256 && (long long)2 * T * k <= 256LL * sms) T *= 2;
+  k_stebz<<<k, T, 0, s>>>(n, d, e2, scal, k, abstol, w, h->ws.status); count_launch();
   CUDA_TRY(cudaGetLastError());
   k_clusters<<<(k + 127) / 128, 128, 0, s>>>(k, w, scal, iscratch); count_launch();
   CUDA_TRY(cudaGetLastError());

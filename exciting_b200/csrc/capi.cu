@@ -692,21 +692,17 @@ int excfv_seceqnsv(excfv_handle* h, int32_t ngp, int32_t ngkmax, const double* g
   const int n = h->st.nstfv;
   CUDA_TRY(cudaMemcpyAsync(ws.Z2, evecfv, sizeof(cplx) * (size_t)nmatmax * n, cudaMemcpyHostToDevice, s));
   CUDA_TRY(cudaMemcpyAsync(h->sv.evalfv, evalfv, sizeof(double) * n, cudaMemcpyHostToDevice, s));
-  double* dw = nullptr;
-  cplx* dv = nullptr;
-  if ((rc = dalloc(&dw, (size_t)2 * n)) || (rc = dalloc(&dv, (size_t)4 * n * n))) {
-    if (dw) cudaFree(dw);
-    return rc;
-  }
+  void* base = nullptr;
+  if ((rc = handle_scratch(h, (size_t)4 * n * n * sizeof(cplx) + 2 * n * sizeof(double), &base))) return rc;
+  cplx* dv = static_cast<cplx*>(base);
+  double* dw = reinterpret_cast<double*>(dv + (size_t)4 * n * n);
   rc = stage_seceqnsv(h, ngp, ws.Z2, nmatmax, h->sv.evalfv, dw, dv);
   if (rc == EXCFV_OK) rc = stage_status(h, n);
   if (rc == EXCFV_OK) {
     cudaMemcpyAsync(evalsv, dw, sizeof(double) * 2 * n, cudaMemcpyDeviceToHost, s);
     cudaMemcpyAsync(evecsv, dv, sizeof(cplx) * 4 * (size_t)n * n, cudaMemcpyDeviceToHost, s);
-    if (cudaStreamSynchronize(s) != cudaSuccess) rc = EXCFV_ERR_CUDA;
   }
-  cudaFree(dw);
-  cudaFree(dv);
+  if (cudaStreamSynchronize(s) != cudaSuccess && rc == EXCFV_OK) rc = EXCFV_ERR_CUDA;
   return rc;
 }
 

@@ -313,6 +313,9 @@ int stage_setup(excfv_handle* h, int nmatp, int ngp, bool mirror_o);
 // generalized eigensolve on ws.H (full) / ws.O (upper) -> evalfv, evecfv
 int stage_solve(excfv_handle* h, int n, int nstfv, double evaltol, double* d_eval,
                 cplx* d_evec, long long ldevec);
+// the standard eigenproblem of the Hermitian matrix in ws.H (both triangles), FP64
+int stage_solve_standard(excfv_handle* h, int n, int nstfv, double evaltol, double* d_eval, cplx* d_evec,
+                         long long ldevec);
 // the solve from C = U^-H H U^-1 onwards (ws.H = C with both triangles,
 // ws.Ui = U^-1 and, in the precision form, C's complex64 copy in ws.T with
 // leading dimension n rounded up to even): what remains of stage_solve

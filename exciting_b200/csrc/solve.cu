@@ -544,7 +544,17 @@ static int solve_front(excfv_handle* h, int n, bool f32copy) {
 }
 
 static int solve_back_fp64(excfv_handle* h, int n, int k, double evaltol, double* d_eval, cplx* d_evec,
-                           long long ldevec);
+                           long long ldevec, bool standard);
+
+// The standard problem C x = e x (C in ws.H, both triangles, leading dimension
+// n; overwritten), in FP64: no Cholesky factor, no reduction to standard form and
+// no back-transform by U^-1.
+int stage_solve_standard(excfv_handle* h, int n, int k, double evaltol, double* d_eval, cplx* d_evec,
+                         long long ldevec) {
+  if (k < 1 || k > n || k > h->ws.kmax) return EXCFV_ERR_ARG;
+  CUDA_TRY(cudaMemsetAsync(h->ws.status, 0, ST_SETUP * sizeof(int), h->stream));
+  return solve_back_fp64(h, n, k, evaltol, d_eval, d_evec, ldevec, true);
+}
 
 int stage_solve(excfv_handle* h, int n, int k, double evaltol, double* d_eval, cplx* d_evec,
                 long long ldevec) {
@@ -606,9 +616,13 @@ static int solve_back_fp64(excfv_handle* h, int n, int k, double evaltol, double
   } else {
     if ((rc = apply_q(h, n, k, ws.H, ld, Z, ld, 1))) return rc;
   }
-  if ((rc = zgemm1(s, OP_N, OP_N, n, k, n, one, ws.Ui, ld, Z, ld, zero, d_evec, ldevec, TRI_NONE,
-                   TRI_UPPER, TRI_NONE)))
+  if (standard) {
+    CUDA_TRY(cudaMemcpy2DAsync(d_evec, sizeof(cplx) * ldevec, Z, sizeof(cplx) * ld, sizeof(cplx) * n, k,
+                               cudaMemcpyDeviceToDevice, s));
+  } else if ((rc = zgemm1(s, OP_N, OP_N, n, k, n, one, ws.Ui, ld, Z, ld, zero, d_evec, ldevec, TRI_NONE,
+                          TRI_UPPER, TRI_NONE))) {
     return rc;
+  }
   prof_end(h, PROF_BACKTR);
   ws.Z = Z;  // cholqr may have swapped the buffers
   k_copy_eval<<<(k + 127) / 128, 128, 0, s>>>(k, ws.w, d_eval); count_launch();

@@ -294,8 +294,7 @@ __global__ void __launch_bounds__(TT + 32, 1)
     const long long ntri = (long long)nt * (nt + 1) / 2;
     const long long t_beg = ntri * bid / G, t_end = ntri * (bid + 1) / G;
     constexpr int BPT = 64 / R::BC;    // TMA tiles (boxes) per 64-column tile
-    constexpr int NPASS = R::BC / 16;  // 16-column passes per box
-    const int rg = tid & 15, cq = tid >> 4;
+      const int rg = tid & 15, cq = tid >> 4;
     double vav_re = 0.0, vav_im = 0.0;
     if (tid == 0) {
       const cplx alpha = ldT(C + (c + 1) + ld * c);
@@ -355,52 +354,69 @@ __global__ void __launch_bounds__(TT + 32, 1)
           for (int u = 0; u < 4; ++u) { xr[u] = s_xr[rg + 16 * u]; xrT[u] = fromD<T2>(xr[u]); }
         }
         const int bend = min(ntile, (g1 - Jb) * BPT);
-        // Two tiles per step: their products and shuffle reductions are
-        // independent, so each warp has two chains in flight.
-        constexpr int NB = 2;
-        for (; b < bend;) {
-          const int nb = min(NB, bend - b);
-          T2 cp[NB][NPASS];
-          int jcol[NB][NPASS];
-          T2 xjv[NB][NPASS];
+        // One 64-column tile (BPT boxes) per step, as four groups of 16 columns:
+        // fused multiply-adds without a test left of the diagonal block, and one
+        // reduction of the four groups' column sums that scatters them over the
+        // lanes (two boxes at a time, each summed over all lanes, spent 0.34 us
+        // per box in the lanes of a batch, this form 0.28 us).
+        constexpr int SPU = R::BC / 16;
+        for (; b < bend; b += BPT) {
+          const int nb = min(BPT, bend - b), nz = nb * SPU;
+          const int jt = Jb + b / BPT;  // column tile of this step
+          const bool diag = (jt == I);
+          const T2* tl[BPT];
 #pragma unroll
-          for (int z = 0; z < NB; ++z) {
-            if (z >= nb) break;
+          for (int z = 0; z < BPT; ++z) {
             const unsigned q = gtile + b + z;
-            mbar_wait(&s_full[q % R::STAGES], (q / R::STAGES) & 1u, a.status, a.wait_ns);
+            if (z < nb) mbar_wait(&s_full[q % R::STAGES], (q / R::STAGES) & 1u, a.status, a.wait_ns);
+            tl[z] = ring + (size_t)(q % R::STAGES) * R::TILE + cq * RCH;
           }
+          const T2* xq = s_x + (jt - g0) * 64 + cq;
+          T2 cp[4];
 #pragma unroll
-          for (int z = 0; z < NB; ++z) {
+          for (int z = 0; z < 4; ++z) cp[z] = fromD<T2>(cmk(0.0, 0.0));
+          if (!diag && nz == 4) {
 #pragma unroll
-            for (int ps = 0; ps < NPASS; ++ps) { cp[z][ps] = fromD<T2>(cmk(0.0, 0.0)); jcol[z][ps] = -1; }
-            if (z >= nb) continue;
-            const int bz = b + z;
-            const T2* tile = ring + (size_t)((gtile + bz) % R::STAGES) * R::TILE;
-            const int jt = Jb + bz / BPT;              // column tile of this box
-            const bool diag = (jt == I);
+            for (int z = 0; z < 4; ++z) {
+              const T2 xj = xq[z * 16];
+              const T2* tile = tl[z / SPU] + (z % SPU) * 16 * RCH;
 #pragma unroll
-            for (int ps = 0; ps < NPASS; ++ps) {
-              const int cb = ps * 16 + cq;              // column within the box
-              const int jl = (bz % BPT) * R::BC + cb;   // column within the 64-wide tile
-              const T2 xj = s_x[(jt - g0) * 64 + jl];
-              xjv[z][ps] = xj;
-              jcol[z][ps] = rb + jt * 64 + jl;
+              for (int u = 0; u < 4; ++u) {
+                const T2 av = tile[rg + 16 * u];
+                if constexpr (sizeof(T2) == 16) {
+                  rowp[u].x = fma(av.x, xj.x, fma(-av.y, xj.y, rowp[u].x));
+                  rowp[u].y = fma(av.x, xj.y, fma(av.y, xj.x, rowp[u].y));
+                } else {
+                  rowf[u].x = fmaf(av.x, xj.x, fmaf(-av.y, xj.y, rowf[u].x));
+                  rowf[u].y = fmaf(av.x, xj.y, fmaf(av.y, xj.x, rowf[u].y));
+                }
+                cp[z].x = mad(av.x, xrT[u].x, mad(av.y, xrT[u].y, cp[z].x));
+                cp[z].y = mad(av.x, xrT[u].y, mad(-av.y, xrT[u].x, cp[z].y));
+              }
+            }
+          } else {
+#pragma unroll
+            for (int z = 0; z < 4; ++z) {
+              if (z >= nz) continue;
+              const T2 xj = xq[z * 16];
+              const T2* tile = tl[z / SPU] + (z % SPU) * 16 * RCH;
+              const int jl = diag ? z * 16 + cq : -1;  // column within the diagonal block
 #pragma unroll
               for (int u = 0; u < 4; ++u) {
                 const int rl = rg + 16 * u;
-                const T2 av = tile[cb * RCH + rl];
-                if (!diag || rl >= jl) {  // row part: A(r, j) x~(j)
+                const T2 av = tile[rl];
+                if (rl >= jl) {  // row part: A(r, j) x~(j)
                   if constexpr (sizeof(T2) == 16) {
-                    rowp[u].x += av.x * xj.x - av.y * xj.y;
-                    rowp[u].y += av.x * xj.y + av.y * xj.x;
+                    rowp[u].x = fma(av.x, xj.x, fma(-av.y, xj.y, rowp[u].x));
+                    rowp[u].y = fma(av.x, xj.y, fma(av.y, xj.x, rowp[u].y));
                   } else {
                     rowf[u].x = fmaf(av.x, xj.x, fmaf(-av.y, xj.y, rowf[u].x));
                     rowf[u].y = fmaf(av.x, xj.y, fmaf(av.y, xj.x, rowf[u].y));
                   }
                 }
-                if (!diag || rl > jl) {   // column part: conj(A(r, j)) x~(r)
-                  cp[z][ps].x += av.x * xrT[u].x + av.y * xrT[u].y;
-                  cp[z][ps].y += av.x * xrT[u].y - av.y * xrT[u].x;
+                if (rl > jl) {   // column part: conj(A(r, j)) x~(r)
+                  cp[z].x = mad(av.x, xrT[u].x, mad(av.y, xrT[u].y, cp[z].x));
+                  cp[z].y = mad(av.x, xrT[u].y, mad(-av.y, xrT[u].x, cp[z].y));
                 }
               }
             }
@@ -413,32 +429,20 @@ __global__ void __launch_bounds__(TT + 32, 1)
           if (lane == 0) {
             for (int z = 0; z < nb; ++z) mbar_arrive(&s_empty[(gtile + b + z) % R::STAGES]);
           }
-#pragma unroll
-          for (int o = 1; o < 16; o <<= 1)
-#pragma unroll
-            for (int z = 0; z < NB; ++z)
-#pragma unroll
-              for (int ps = 0; ps < NPASS; ++ps) {
-                cp[z][ps].x += __shfl_xor_sync(0xffffffffu, cp[z][ps].x, o);
-                cp[z][ps].y += __shfl_xor_sync(0xffffffffu, cp[z][ps].y, o);
-              }
-          if (rg == 0) {
-#pragma unroll
-            for (int z = 0; z < NB; ++z)
-#pragma unroll
-              for (int ps = 0; ps < NPASS; ++ps) {
-                const int j = jcol[z][ps];
-                if (j >= r0g && j < n) {
-                  const cplx sc = cmul(scale, toD(cp[z][ps]));
-                  atomicAdd(&ycur[j].x, sc.x);
-                  atomicAdd(&ycur[j].y, sc.y);
-                  const cplx vj = (j == c + 1) ? cmk(1.0, 0.0) : cmul(toD(xjv[z][ps]), scale);
-                  vav_re += vj.x * sc.x + vj.y * sc.y;  // conj(v_j) * contribution
-                  vav_im += vj.x * sc.y - vj.y * sc.x;
-                }
-              }
+          const T2 kk = scatter_sum16(cp, lane);
+          const int z = 2 * ((lane >> 3) & 1) + ((lane >> 2) & 1);
+          const int j = rb + jt * 64 + z * 16 + cq;
+          if ((lane & 3) < 2 && z < nz && j >= r0g && j < n) {
+            const cplx sc = cmul(scale, toD(kk));
+            if (lane & 1) {
+              atomicAdd(&ycur[j].y, sc.y);
+            } else {
+              atomicAdd(&ycur[j].x, sc.x);
+              const cplx vj = (j == c + 1) ? cmk(1.0, 0.0) : cmul(toD(xq[z * 16]), scale);
+              vav_re += vj.x * sc.x + vj.y * sc.y;  // conj(v_j) * contribution
+              vav_im += vj.x * sc.y - vj.y * sc.x;
+            }
           }
-          b += nb;
         }
         if constexpr (sizeof(T2) == 8) {
 #pragma unroll

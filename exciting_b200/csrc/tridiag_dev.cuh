@@ -138,6 +138,32 @@ __device__ __forceinline__ cplx shfl4_sum(cplx v) {
   return v;
 }
 
+__device__ __forceinline__ double mad(double a, double b, double c) { return fma(a, b, c); }
+__device__ __forceinline__ float mad(float a, float b, float c) { return fmaf(a, b, c); }
+
+// Sums of four column groups over the 16 lanes of a half warp, scattered: lane
+// bits 3 and 2 select the group whose sum the lane ends up with.
+template <typename T2>
+__device__ __forceinline__ T2 scatter_sum16(const T2 (&cp)[4], int lane) {
+  const bool h3 = (lane >> 3) & 1, h2 = (lane >> 2) & 1;
+  const T2 s0 = h3 ? cp[0] : cp[2], s1 = h3 ? cp[1] : cp[3];
+  T2 k0 = h3 ? cp[2] : cp[0], k1 = h3 ? cp[3] : cp[1];
+  k0.x += __shfl_xor_sync(0xffffffffu, s0.x, 8);
+  k0.y += __shfl_xor_sync(0xffffffffu, s0.y, 8);
+  k1.x += __shfl_xor_sync(0xffffffffu, s1.x, 8);
+  k1.y += __shfl_xor_sync(0xffffffffu, s1.y, 8);
+  T2 kk = h2 ? k1 : k0;
+  const T2 s2 = h2 ? k0 : k1;
+  kk.x += __shfl_xor_sync(0xffffffffu, s2.x, 4);
+  kk.y += __shfl_xor_sync(0xffffffffu, s2.y, 4);
+#pragma unroll
+  for (int o = 2; o > 0; o >>= 1) {
+    kk.x += __shfl_xor_sync(0xffffffffu, kk.x, o);
+    kk.y += __shfl_xor_sync(0xffffffffu, kk.y, o);
+  }
+  return kk;
+}
+
 // a * conj(b)
 __device__ __forceinline__ cplx cmul_cb(cplx a, cplx b) {
   return cmk(a.x * b.x + a.y * b.y, a.y * b.x - a.x * b.y);

@@ -213,9 +213,6 @@ __device__ __forceinline__ int col_at(int I, int j) {  // column part of block r
   return 32 * I * (I + 1) + j;
 }
 
-__device__ __forceinline__ double mad(double a, double b, double c) { return fma(a, b, c); }
-__device__ __forceinline__ float mad(float a, float b, float c) { return fmaf(a, b, c); }
-
 // ---------------------------------------------------------------------------
 template <typename T2>
 __device__ void flow_worker(const FlowArgs<T2>& a, const CUtensorMap* tmap, unsigned char* dsm, int w) {
@@ -449,31 +446,8 @@ __device__ void flow_worker(const FlowArgs<T2>& a, const CUtensorMap* tmap, unsi
           sl -= a.stages;
           ++wrap;
         }
-        // sum over the 16 rows groups of the half warp, scattering the four
-        // column groups: lane bits 3 and 2 select the group it ends up with
-        const bool h3 = (lane >> 3) & 1, h2 = (lane >> 2) & 1;
-        T2 k0, k1;
-        {
-          const T2 s0 = h3 ? cp[0] : cp[2], s1 = h3 ? cp[1] : cp[3];
-          k0 = h3 ? cp[2] : cp[0];
-          k1 = h3 ? cp[3] : cp[1];
-          k0.x += __shfl_xor_sync(0xffffffffu, s0.x, 8);
-          k0.y += __shfl_xor_sync(0xffffffffu, s0.y, 8);
-          k1.x += __shfl_xor_sync(0xffffffffu, s1.x, 8);
-          k1.y += __shfl_xor_sync(0xffffffffu, s1.y, 8);
-        }
-        T2 kk = h2 ? k1 : k0;
-        {
-          const T2 s0 = h2 ? k0 : k1;
-          kk.x += __shfl_xor_sync(0xffffffffu, s0.x, 4);
-          kk.y += __shfl_xor_sync(0xffffffffu, s0.y, 4);
-        }
-#pragma unroll
-        for (int o = 2; o > 0; o >>= 1) {
-          kk.x += __shfl_xor_sync(0xffffffffu, kk.x, o);
-          kk.y += __shfl_xor_sync(0xffffffffu, kk.y, o);
-        }
-        const int z = 2 * (int)h3 + (int)h2;
+        const T2 kk = scatter_sum16(cp, lane);
+        const int z = 2 * ((lane >> 3) & 1) + ((lane >> 2) & 1);
         const int j = b0 * BC + (q0 + z) * 16 + cq;
         if ((lane & 3) == 0 && z < nz && j > i && j < nrel) stw(cw + j, toD(kk), tag);
         if constexpr (sizeof(T2) == 8) {  // FP32 row sums of at most 32 terms

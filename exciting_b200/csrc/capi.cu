@@ -2,6 +2,7 @@
 // data upload, workspace, and the drop-ins for match / hamiltonandoverlapsetup
 // / solvewithlapack / seceqnfv / seceqn.
 #include <cstdarg>
+#include <type_traits>
 #include <cstring>
 #include <vector>
 #include <chrono>
@@ -122,20 +123,9 @@ void free_static(DevStatic& st) {
 }
 
 void free_workspace(Workspace& ws) {
-  dfree(ws.H); dfree(ws.O); dfree(ws.Ui); dfree(ws.T); dfree(ws.Apk); dfree(ws.Zpk);
-  dfree(ws.ylm); dfree(ws.djl); dfree(ws.apwalm); dfree(ws.igpig); dfree(ws.vgpc); dfree(ws.gpc);
-  dfree(ws.tpgpc); dfree(ws.sfacgp); dfree(ws.gk_iv); dfree(ws.d); dfree(ws.e); dfree(ws.tau);
-  dfree(ws.Wp); dfree(ws.red); dfree(ws.w); dfree(ws.stein_ws); dfree(ws.icl); dfree(ws.ybuf);
-  dfree(ws.Z); dfree(ws.Z2); dfree(ws.Gk); dfree(ws.Gki); dfree(ws.Tf); dfree(ws.Xs);
-  dfree(ws.status); dfree(ws.bar); dfree(ws.part); dfree(ws.prog);
-  if (ws.flow) cudaFree(ws.flow);
-  ws.flow = nullptr; dfree(ws.slices); dfree(ws.slice_sc);
-  ws.slices_elems = ws.slice_sc_n = 0;
+  if (ws.block) cudaFree(ws.block);
   if (ws.h_pinned) cudaFreeHost(ws.h_pinned);
-  ws.h_pinned = nullptr;
-  ws.h_pinned_bytes = 0;
-  ws.part_cap = 0;
-  ws.nmatmax = ws.ngkmax = ws.kmax = 0;
+  ws = Workspace();
 }
 
 int handle_scratch(excfv_handle* h, size_t bytes, void** p) {
@@ -360,41 +350,44 @@ int stage_reserve(excfv_handle* h, int nmatmax, int ngkmax, int kmax) {
   const DevStatic& st = h->st;
   const size_t n = nmatmax, n2 = n * n, AM = (size_t)st.natmtot * st.maxaa;
   const size_t K = kmax;
-  int rc;
-  if ((rc = dalloc(&ws.H, n2)) || (rc = dalloc(&ws.O, n2)) || (rc = dalloc(&ws.Ui, n2)) ||
-      (rc = dalloc(&ws.T, n2)) || (rc = dalloc(&ws.Apk, AM * ngkmax)) ||
-      (rc = dalloc(&ws.Zpk, AM * ngkmax)) || (rc = dalloc(&ws.ylm, (size_t)st.lmmaxapw * ngkmax)) ||
-      (rc = dalloc(&ws.djl, (size_t)ngkmax * (st.lmaxapw + 1) * st.apwordmax * st.nspecies)) ||
-      (rc = dalloc(&ws.apwalm, (size_t)ngkmax * st.apwordmax * st.lmmaxapw * st.natmtot)) ||
-      (rc = dalloc(&ws.igpig, (size_t)ngkmax)) || (rc = dalloc(&ws.vgpc, (size_t)3 * ngkmax)) ||
-      (rc = dalloc(&ws.gpc, (size_t)ngkmax)) || (rc = dalloc(&ws.tpgpc, (size_t)2 * ngkmax)) ||
-      (rc = dalloc(&ws.sfacgp, (size_t)ngkmax * st.natmtot)) ||
-      (rc = dalloc(&ws.gk_iv, (size_t)3 * ngkmax)) || (rc = dalloc(&ws.d, n)) ||
-      (rc = dalloc(&ws.e, n)) || (rc = dalloc(&ws.tau, n)) ||
-      (rc = dalloc(&ws.Wp, n * 4 * tridiag_nb())) ||
-      (rc = dalloc(&ws.red, (size_t)tridiag_workspace_doubles())) || (rc = dalloc(&ws.w, n)) ||
-      (rc = dalloc(&ws.stein_ws, tridiag_eig_scratch_doubles((int)n, (int)K))) ||
-      (rc = dalloc(&ws.icl, K)) || (rc = dalloc(&ws.ybuf, 2 * n)) || (rc = dalloc(&ws.Z, n * K)) ||
-      (rc = dalloc(&ws.Z2, n * K)) || (rc = dalloc(&ws.Gk, K * K)) || (rc = dalloc(&ws.Gki, K * K)) ||
-      (rc = dalloc(&ws.Tf, backtr_factor_elems((int)n))) || (rc = dalloc(&ws.Xs, 2 * 256 * K)) ||
-      (rc = dalloc(&ws.status, (size_t)ST_NWORDS)) || (rc = dalloc(&ws.bar, (size_t)4)) ||
-      (rc = dalloc(&ws.prog, n)) ||
-      (rc = dalloc(reinterpret_cast<unsigned char**>(&ws.flow), tridiag_flow_bytes((int)n, h->nsm))) ||
-      (rc = dalloc(&ws.part, std::max((size_t)(8u << 20), n * 64 * 4)))) {
-    free_workspace(ws);
-    return rc;
-  }
-  ws.part_cap = std::max((size_t)(8u << 20), n * 64 * 4);
-  if (want_slices) {
-    // A and aa A as BF16 slice planes (setup_bf16.cu)
-    const size_t pe = bf16x_plane_elems((int)AM, (int)ngkmax);
-    const size_t nsc = 2 * (size_t)bf16x_rpad((int)ngkmax);
-    if ((rc = dalloc(&ws.slices, pe)) || (rc = dalloc(&ws.slice_sc, nsc))) {
-      free_workspace(ws);
-      return rc;
+  // split-K scratch: up to 16 partial products of an n x n result, 8 M elements
+  // at most, and the back-transform's needs
+  ws.part_cap = std::max(std::min((size_t)(8u << 20), 16 * n2), n * 64 * 4);
+  // the slices of the precision form: A and aa A as BF16 slice planes (setup_bf16.cu)
+  ws.slices_elems = want_slices ? bf16x_plane_elems((int)AM, (int)ngkmax) : 0;
+  ws.slice_sc_n = want_slices ? 2 * (size_t)bf16x_rpad((int)ngkmax) : 0;
+  // All arrays in one allocation: two passes over the list, sizes and then
+  // addresses (first call of a batch of 28 k-points of order ~300: 38.9 ms with an
+  // allocation per array and 8 lanes, 24.7 ms like this with 28).
+  size_t total = 0;
+  for (int pass = 0; pass < 2; ++pass) {
+    if (pass) {
+      const int rc = dalloc(&ws.block, total);
+      if (rc) {
+        free_workspace(ws);
+        return rc;
+      }
     }
-    ws.slices_elems = pe;
-    ws.slice_sc_n = nsc;
+    size_t at = 0;
+    auto take = [&](auto** p, size_t count) {
+      if (pass) *p = count ? reinterpret_cast<std::remove_reference_t<decltype(*p)>>(ws.block + at) : nullptr;
+      at += (count * sizeof(**p) + 255) / 256 * 256;
+    };
+    take(&ws.H, n2); take(&ws.O, n2); take(&ws.Ui, n2); take(&ws.T, n2);
+    take(&ws.Apk, AM * ngkmax); take(&ws.Zpk, AM * ngkmax);
+    take(&ws.ylm, (size_t)st.lmmaxapw * ngkmax);
+    take(&ws.djl, (size_t)ngkmax * (st.lmaxapw + 1) * st.apwordmax * st.nspecies);
+    take(&ws.apwalm, (size_t)ngkmax * st.apwordmax * st.lmmaxapw * st.natmtot);
+    take(&ws.igpig, (size_t)ngkmax); take(&ws.vgpc, (size_t)3 * ngkmax); take(&ws.gpc, (size_t)ngkmax);
+    take(&ws.tpgpc, (size_t)2 * ngkmax); take(&ws.sfacgp, (size_t)ngkmax * st.natmtot);
+    take(&ws.gk_iv, (size_t)3 * ngkmax); take(&ws.d, n); take(&ws.e, n); take(&ws.tau, n);
+    take(&ws.Wp, n * 4 * tridiag_nb()); take(&ws.red, (size_t)tridiag_workspace_doubles()); take(&ws.w, n);
+    take(&ws.stein_ws, tridiag_eig_scratch_doubles((int)n, (int)K)); take(&ws.icl, K); take(&ws.ybuf, 2 * n);
+    take(&ws.Z, n * K); take(&ws.Z2, n * K); take(&ws.Gk, K * K); take(&ws.Gki, K * K);
+    take(&ws.Tf, backtr_factor_elems((int)n)); take(&ws.Xs, 2 * 256 * K); take(&ws.status, (size_t)ST_NWORDS);
+    take(&ws.bar, (size_t)4); take(&ws.prog, n); take(&ws.flow, tridiag_flow_bytes((int)n, h->nsm));
+    take(&ws.part, ws.part_cap); take(&ws.slices, ws.slices_elems); take(&ws.slice_sc, ws.slice_sc_n);
+    total = at;
   }
   // zeroed in the handle's stream order (lane streams do not wait for the legacy stream)
   CUDA_TRY(cudaMemsetAsync(ws.status, 0, ST_NWORDS * sizeof(int), h->stream));
@@ -1684,11 +1677,16 @@ static BatchArgs make_batch(int32_t nk, const int32_t* nmatp, const int32_t* ngp
   return b;
 }
 
+// Lanes of a batch when the caller has chosen none.  Orders that the cluster
+// kernel reduces alone in clusters of 8 have no cooperative panels to share the
+// SMs out to: up to 32 lanes, all k-points of most batches at once (28 k-points of
+// order ~300: 8 lanes 10.5 ms, 16 8.9, 28 6.1).
 static int default_lanes(excfv_handle* h, const BatchArgs& b) {
   if (h->nlanes_pref > 0) return h->nlanes_pref;
   int nmax = 0;
   for (int k = 0; k < b.nk; ++k) nmax = std::max(nmax, (int)b.nmatp[k]);
-  return std::min(8, max_lanes_for(h, nmax));
+  const int most = nmax <= tridiag_tail_lane_max(h->prec == EXCFV_PREC_MIXED) ? 32 : 8;
+  return std::min(most, max_lanes_for(h, nmax));
 }
 
 int excfv_seceqn_batched_dev(excfv_handle* h, int32_t nk, const int32_t* nmatp, const int32_t* ngp,

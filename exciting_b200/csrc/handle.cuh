@@ -56,6 +56,7 @@ struct DevStatic {
 };
 
 struct Workspace {
+  unsigned char* block = nullptr;  // the allocation that holds every array below
   int nmatmax = 0, ngkmax = 0, kmax = 0;
   cplx* H = nullptr;        // n x n
   cplx* O = nullptr;        // n x n
@@ -93,7 +94,7 @@ struct Workspace {
   size_t part_cap = 0;      // complex elements
   int* status = nullptr;    // ST_NWORDS
   unsigned int* bar = nullptr;  // grid barrier words
-  void* flow = nullptr;     // words of the dataflow panel kernel (tridiag_flow.cu)
+  unsigned char* flow = nullptr;  // words of the dataflow panel kernel (tridiag_flow.cu)
   int* prog = nullptr;      // (n) per-sweep progress of the band -> tridiagonal chase
   // split-BF16 setup of the precision form: slice planes of A and of aa A, row scales
   __nv_bfloat16* slices = nullptr;
@@ -354,6 +355,8 @@ int tridiag_rows_per_cta(bool complex64);
 // the first column of an n x n reduction that goes to the cluster kernel of
 // the last columns (tridiag_tail.cu); n - 1 when the panels take them all
 int tridiag_tail_start(int n, bool complex64, int G);
+// the largest order that a lane of a batch reduces in one cluster of 8 (tridiag_tail.cu)
+int tridiag_tail_lane_max(bool complex64);
 // elements of ws.Tf the back-transform needs for nrefl reflectors: the Gram
 // matrices and block-reflector factors of 256-wide blocks and their merge
 // scratch (solve.cu); ws.Xs holds 2 x 256 x kmax

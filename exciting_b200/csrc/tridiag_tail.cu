@@ -388,12 +388,19 @@ int tridiag_tail_max() {
 template int tridiag_tail_max<double2>();
 template int tridiag_tail_max<float2>();
 
+int tridiag_tail_lane_max(bool complex64) { return complex64 ? tail_max_cl<float2, 8>() : tail_max_cl<double2, 8>(); }
+
 // reduces the trailing block C(c0:n, c0:n) (lower triangle, already updated
 // by the panels before c0) and leaves reflectors, d, e, tau as the panels do
 template <typename T2>
 int tridiag_tail(excfv_handle* h, int n, int c0, T2* C, long long ld) {
   if (n - c0 < 2) return EXCFV_ERR_ARG;
-  return tail_cluster() == 16 ? tail_launch<T2, 16>(h, n, c0, C, ld) : tail_launch<T2, 8>(h, n, c0, C, ld);
+  // Lanes of a batch share the GPU: twice as many clusters of 8 run at once, and
+  // one takes little longer on the blocks it holds (28 k-points of order ~300 on
+  // 28 lanes 6.1 against 8.6 ms).
+  const bool small = h->grid_ctas > 0 && n - c0 <= tail_max_cl<T2, 8>();
+  if (small || tail_cluster() != 16) return tail_launch<T2, 8>(h, n, c0, C, ld);
+  return tail_launch<T2, 16>(h, n, c0, C, ld);
 }
 template int tridiag_tail<double2>(excfv_handle*, int, int, double2*, long long);
 template int tridiag_tail<float2>(excfv_handle*, int, int, float2*, long long);

@@ -178,6 +178,14 @@ __global__ void __launch_bounds__(GT) k_zgemm_cn_tma(TmaGemmArgs a, const __grid
   if (tid == 0)
     for (int it = 0; it < STAGES && it < nit; ++it) issue(it);
 
+  cplx* C = z ? a.C1 : a.C0;
+  const bool use_beta = a.splitk <= 1 && (a.beta.x != 0.0 || a.beta.y != 0.0);
+  if (use_beta)  // the C tile on its way to L2 during the products
+    for (int q = tid; q < TM / 8 * TN; q += GT) {
+      const int row = i0 + q % (TM / 8) * 8, col = j0 + q / (TM / 8);
+      if (row < a.m && col < a.n) asm volatile("prefetch.global.L2 [%0];" ::"l"(C + row + a.ldc * col));
+    }
+
   const int wm = (warp & 1) * 32, wn = (warp >> 1) * 32;
   double acc[4][4][2][2];
 #pragma unroll
@@ -245,23 +253,32 @@ __global__ void __launch_bounds__(GT) k_zgemm_cn_tma(TmaGemmArgs a, const __grid
     }
     return;
   }
-  cplx* C = z ? a.C1 : a.C0;
-  const bool use_beta = (a.beta.x != 0.0 || a.beta.y != 0.0);
+  // C is read eight entries at a time before the first of their stores (a load does
+  // not pass a store that may alias it; order 5028, setup and the rank-64 updates of
+  // the Cholesky factor: 33.7 -> 28.7 ms with this and one launch per update)
 #pragma unroll
   for (int x = 0; x < 4; ++x) {
     const int row = i0 + wm + 8 * x + (lane >> 2);
     if (row >= a.m) continue;
+    cplx old[4][2];
+    if (use_beta) {
+#pragma unroll
+      for (int y = 0; y < 4; ++y)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int col = j0 + wn + 8 * y + (lane & 3) * 2 + e;
+          if (col < a.n && !(a.uplo == TRI_UPPER && row > col)) old[y][e] = C[row + a.ldc * col];
+        }
+    }
 #pragma unroll
     for (int y = 0; y < 4; ++y)
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
         const int col = j0 + wn + 8 * y + (lane & 3) * 2 + e;
-        if (col >= a.n) continue;
-        if (a.uplo == TRI_UPPER && row > col) continue;
+        if (col >= a.n || (a.uplo == TRI_UPPER && row > col)) continue;
         cplx out = cmul(a.alpha, cmk(acc[x][y][0][e], acc[x][y][1][e]));
-        cplx* dst = C + row + a.ldc * col;
-        if (use_beta) out = cadd(out, cmul(a.beta, *dst));
-        *dst = out;
+        if (use_beta) out = cadd(out, cmul(a.beta, old[y][e]));
+        C[row + a.ldc * col] = out;
       }
   }
 }
@@ -274,7 +291,7 @@ __global__ void k_split_reduce(TmaGemmArgs a) {
   tile_coords(a, t, z, ti, tj);
   cplx* C = z ? a.C1 : a.C0;
   const bool use_beta = (a.beta.x != 0.0 || a.beta.y != 0.0);
-  for (int e = threadIdx.x; e < TM * TN; e += blockDim.x) {
+  for (int e = blockIdx.y * blockDim.x + threadIdx.x; e < TM * TN; e += gridDim.y * blockDim.x) {
     const int r = e % TM, c = e / TM;
     const int row = ti * TM + r, col = tj * TN + c;
     if (row >= a.m || col >= a.n) continue;
@@ -359,24 +376,25 @@ int zgemm_cn_tma(excfv_handle* h, int m, int n, int k, cplx alpha, const cplx* c
   const int budget = (h->grid_ctas > 0) ? h->grid_ctas : h->nsm;
   const long long R = (long long)std::max(1, per_sm) * budget;  // resident CTAs
   const long long total = (long long)a.tpb * batch;
-  const long long full = (total / R) * R;
+  // the K pieces of the last wave's tiles; in one piece (K < 128) all tiles go in one
+  // launch, since a launch of its own leaves SMs idle before it and after
+  const GemmCtx& g = gemm_ctx();
+  long long rem = total % R;
+  int sk = (rem > 0) ? (int)std::max(1LL, std::min<long long>(R / rem, a.nk / 4)) : 1;
+  while (sk > 1 && (size_t)rem * sk * TM * TN > g.cap) --sk;
+  if (sk == 1) rem = 0;
+  const long long full = total - rem;
   if (full > 0) {
     a.tile0 = 0; a.splitk = 1; a.part = nullptr;
     k_zgemm_cn_tma<<<(unsigned)full, GT, smem, s>>>(a, mA[0], mA[1], mB[0], mB[1]); count_launch();
     CUDA_TRY(cudaGetLastError());
   }
-  const long long rem = total - full;
   if (rem > 0) {
-    const GemmCtx& g = gemm_ctx();
-    int sk = (int)std::max(1LL, std::min<long long>(R / rem, a.nk / 4));
-    while (sk > 1 && (size_t)rem * sk * TM * TN > g.cap) --sk;
-    a.tile0 = (int)full; a.splitk = sk; a.part = (sk > 1) ? g.ws : nullptr;
+    a.tile0 = (int)full; a.splitk = sk; a.part = g.ws;
     k_zgemm_cn_tma<<<(unsigned)(rem * sk), GT, smem, s>>>(a, mA[0], mA[1], mB[0], mB[1]); count_launch();
     CUDA_TRY(cudaGetLastError());
-    if (sk > 1) {
-      k_split_reduce<<<(unsigned)rem, 256, 0, s>>>(a); count_launch();
-      CUDA_TRY(cudaGetLastError());
-    }
+    k_split_reduce<<<dim3((unsigned)rem, 4), 256, 0, s>>>(a); count_launch();
+    CUDA_TRY(cudaGetLastError());
   }
   return EXCFV_OK;
 }

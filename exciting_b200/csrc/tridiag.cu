@@ -5,8 +5,9 @@
 // blocked ZHETRD, restated): one persistent cooperative kernel reduces the
 // NBT columns of a panel, then one GEMM applies the rank-2*NBT update
 // C22 -= [V W] [W V]^H to the lower triangle of the trailing matrix (the only
-// part the reduction reads).  Inside the panel kernel every column costs two
-// grid-wide barriers:
+// part the reduction reads).  A handle with the whole GPU runs its panels as a
+// dataflow between thread blocks (tridiag_flow.cu); the kernel here, for the lanes
+// of a batch and as the fallback, costs two grid-wide barriers per column:
 //
 //   phase 1 (row owners)  finish W(:, i-1); update column c with the panel's
 //                         previous reflectors; partial |x|^2 for the norm

@@ -15,22 +15,24 @@
 //   S1  x = C22(c+1:m, c) has arrived in every CTA
 //   B   one warp of every CTA: |x(c+2:m)|^2, beta, tau, scale by ZLARFG (the
 //       panel kernel's formulas; the same operands and order everywhere, so
-//       the same bits), e(c), tau(c); then v = [1; scale x] into vbuf and
-//       into column c of own packed rows (unit entry explicit)
-//   C   y = C22 v: the row part of own rows (a warp per row), the column part
-//       sum_{own i > j} conj(C22_ij) v_i (a thread per column j, no atomics)
+//       the same bits), e(c), tau(c)
+//   C   beside it, C22 x' with x' = x(c+2:m), which needs no reflector: the row
+//       part of own rows (a warp per row), the column part
+//       sum_{own i > j} conj(C22_ij) x'_i (a thread per column j, no atomics)
 //       pushed to the owner of row j
 //   S2
-//   D   owners: y_i = row part + the CL column parts; w0_i = tau y_i to all,
-//       and Re(v^H y) over own rows to all
+//   D   owners: y = C22 v = C22(:, c+1) + scale C22 x'; w0_i = tau y_i to all, and
+//       Re(v^H y) over own rows to all; v = [1; scale x'] into vbuf and into
+//       column c of own packed rows (unit entry explicit)
 //   S3
 //   E   every CTA: alpha = -|tau|^2/2 v^H C22 v from the CL partials (the
-//       panel kernel's real form), w = w0 + alpha v once per entry,
-//       C22 -= v w^H + w v^H on own rows (the diagonal kept real, apart from
-//       the off-diagonal loop); the updated column c+1 goes out at once: x of
+//       panel kernel's real form), C22 -= v w0^H + (w0 + 2 alpha v) v^H on own
+//       rows (the diagonal kept real, apart from the off-diagonal loop); the updated column c+1 goes out at once: x of
 //       the next column and d(c+1)
 //
-// with three cluster barriers per column.  All CTAs run the same loop, so
+// with three cluster barriers per column.  With the reflector and v formed before
+// the products a column took 5.1 us at order 316 and 3.9 at 86; like this 4.2 and
+// 3.0 us.  All CTAs run the same loop, so
 // every barrier is reached by all of them; the kernel has no other waits.
 // The reflectors, d, e and tau it leaves are those of the panel kernel's
 // convention, so the back-transform reads them unchanged.
@@ -73,7 +75,7 @@ __global__ void __launch_bounds__(TT, 1) k_tridiag_tail(int n, int c0, T2* C, lo
   // map_shared_rank address keeps the offset); the packed rows come last.
   cplx* xbuf = reinterpret_cast<cplx*>(dsm);     // column c below the diagonal (pushed)
   cplx* vbuf = xbuf + m;                         // the reflector (local)
-  cplx* wbuf = vbuf + m;                         // w0 = tau y (pushed by the row owners), then w
+  cplx* wbuf = vbuf + m;                         // w0 = tau y (pushed by the row owners)
   cplx* ypart = wbuf + m;                        // [CL][smax]: column parts for own rows (pushed)
   cplx* yrow = ypart + (size_t)CL * smax;        // row parts of own rows (local)
   cplx* tau_loc = yrow + smax;                   // tau(c) of the columns c = rank mod CL (local)
@@ -108,10 +110,10 @@ __global__ void __launch_bounds__(TT, 1) k_tridiag_tail(int n, int c0, T2* C, lo
 
   for (int c = 0; c < m - 1; ++c) {
     cl.sync();  // x of column c has arrived
-    // ---- the reflector (one warp; every CTA derives the same bits from the
-    //      same operands: |x(c+2:)|^2 summed in the same order), v into vbuf
-    //      and into the packed rows ------------------------------------------
-    if (warp == 0) {
+    // ---- the reflector (the last warp, beside the products; every CTA derives
+    //      the same bits from the same operands: |x(c+2:)|^2 summed in the same
+    //      order) --------------------------------------------------------------
+    if (warp == NW - 1) {
       double xn2 = 0.0;
       for (int i = c + 2 + lane; i < m; i += 32) {
         const cplx x = xbuf[i];
@@ -140,36 +142,25 @@ __global__ void __launch_bounds__(TT, 1) k_tridiag_tail(int n, int c0, T2* C, lo
         }
       }
     }
-    __syncthreads();
-    const cplx tau = cmk(s_scal[0], s_scal[1]), scale = cmk(s_scal[2], s_scal[3]);
-    // v also replaces column c of own packed rows (dead from here on): the
-    // reflectors go to C once, at the end, so no global store is pending at a
-    // cluster barrier
-    for (int i = c + 1 + tid; i < m; i += TT) {
-      const cplx v = (i == c + 1) ? cmk(1.0, 0.0) : cmul(xbuf[i], scale);
-      vbuf[i] = v;
-      if (i % CL == rank) stT(A + row_off<CL>(rank, i / CL) + c, v);  // unit entry explicit
-    }
-    __syncthreads();
     // own rows from slot s_lo on are the rows >= c + 1
     const int s_lo = (c + 1 > rank) ? (c + 1 - rank + CL - 1) / CL : 0;
-    // ---- y = C22 v: the row part of own rows (a warp per row) ---------------
+    // ---- C22 x' with x' = x(c+2:): the row part of own rows (a warp per row) --
     for (int s = s_lo + warp; s < nslot; s += NW) {
       const int i = rank + CL * s;
       const T2* row = A + row_off<CL>(rank, s);
       // two independent chains per lane
       double ar = 0.0, ai = 0.0, br = 0.0, bi = 0.0;
-      int j = c + 1 + lane;
+      int j = c + 2 + lane;
       for (; j + 32 < i; j += 64) {
-        const cplx a0 = ldT(row + j), v0 = vbuf[j];
-        const cplx a1 = ldT(row + j + 32), v1 = vbuf[j + 32];
+        const cplx a0 = ldT(row + j), v0 = xbuf[j];
+        const cplx a1 = ldT(row + j + 32), v1 = xbuf[j + 32];
         ar += a0.x * v0.x - a0.y * v0.y;
         ai += a0.x * v0.y + a0.y * v0.x;
         br += a1.x * v1.x - a1.y * v1.y;
         bi += a1.x * v1.y + a1.y * v1.x;
       }
       if (j < i) {
-        const cplx a0 = ldT(row + j), v0 = vbuf[j];
+        const cplx a0 = ldT(row + j), v0 = xbuf[j];
         ar += a0.x * v0.x - a0.y * v0.y;
         ai += a0.x * v0.y + a0.y * v0.x;
       }
@@ -181,11 +172,11 @@ __global__ void __launch_bounds__(TT, 1) k_tridiag_tail(int n, int c0, T2* C, lo
       }
       if (lane == 0) {
         const double aii = ldT(row + i).x;
-        const cplx vi = vbuf[i];
-        yrow[s] = cmk(ar + aii * vi.x, ai + aii * vi.y);
+        const cplx xi = (i > c + 1) ? xbuf[i] : cmk(0.0, 0.0);
+        yrow[s] = cmk(ar + aii * xi.x, ai + aii * xi.y);
       }
     }
-    // ---- and the column part: sum over own rows i > j of conj(A_ij) v_i, a
+    // ---- and the column part: sum over own rows i > j of conj(A_ij) x_i, a
     //      thread per column j, pushed to the owner of row j -----------------
     for (int j = c + 1 + tid; j < m; j += TT) {
       int s = (j >= rank) ? (j - rank) / CL + 1 : 0;  // first own row below j
@@ -194,8 +185,8 @@ __global__ void __launch_bounds__(TT, 1) k_tridiag_tail(int n, int c0, T2* C, lo
       for (; s + 1 < nslot; s += 2) {
         const int i0 = rank + CL * s, i1 = i0 + CL;
         const long long o1 = o + i0 + 1;
-        const cplx a0 = ldT(A + o + j), v0 = vbuf[i0];
-        const cplx a1 = ldT(A + o1 + j), v1 = vbuf[i1];
+        const cplx a0 = ldT(A + o + j), v0 = xbuf[i0];
+        const cplx a1 = ldT(A + o1 + j), v1 = xbuf[i1];
         ar += a0.x * v0.x + a0.y * v0.y;
         ai += a0.x * v0.y - a0.y * v0.x;
         br += a1.x * v1.x + a1.y * v1.y;
@@ -204,50 +195,63 @@ __global__ void __launch_bounds__(TT, 1) k_tridiag_tail(int n, int c0, T2* C, lo
       }
       if (s < nslot) {
         const int i0 = rank + CL * s;
-        const cplx a0 = ldT(A + o + j), v0 = vbuf[i0];
+        const cplx a0 = ldT(A + o + j), v0 = xbuf[i0];
         ar += a0.x * v0.x + a0.y * v0.y;
         ai += a0.x * v0.y - a0.y * v0.x;
       }
       cl.map_shared_rank(ypart, j % CL)[rank * smax + j / CL] = cmk(ar + br, ai + bi);
     }
     cl.sync();
-    // ---- own rows: y = row part + every rank's column part; w0 = tau y to
-    //      every CTA (a thread per row and target) -----------------------------
+    const cplx tau = cmk(s_scal[0], s_scal[1]), scale = cmk(s_scal[2], s_scal[3]);
+    // ---- own rows: y = C22 v = C22 e1 + scale (row part + every rank's column
+    //      part); w0 = tau y to every CTA (a thread per row and target) ---------
+    auto y_of = [&](int s) {
+      cplx y = yrow[s], p[4] = {};  // four chains
+#pragma unroll
+      for (int q = 0; q < CL; ++q) p[q & 3] = cadd(p[q & 3], ypart[q * smax + s]);
+      y = cadd(y, cadd(cadd(p[0], p[1]), cadd(p[2], p[3])));
+      cplx a = ldT(A + row_off<CL>(rank, s) + c + 1);
+      if (rank + CL * s == c + 1) a.y = 0.0;
+      return cadd(cmul(scale, y), a);
+    };
     for (int t = s_lo * CL + tid; t < nslot * CL; t += TT) {
       const int s = t / CL, r = t % CL;
-      cplx y = yrow[s];
-      for (int q = 0; q < CL; ++q) y = cadd(y, ypart[q * smax + s]);
-      cl.map_shared_rank(wbuf, r)[rank + CL * s] = cmul(tau, y);
+      cl.map_shared_rank(wbuf, r)[rank + CL * s] = cmul(tau, y_of(s));
     }
     // and the last warp: Re(v^H y) over own rows to every CTA
     if (warp == NW - 1) {
       double vy = 0.0;
       for (int s = s_lo + lane; s < nslot; s += 32) {
-        cplx y = yrow[s];
-        for (int q = 0; q < CL; ++q) y = cadd(y, ypart[q * smax + s]);
-        const cplx v = vbuf[rank + CL * s];
+        const int i = rank + CL * s;
+        const cplx y = y_of(s), v = (i == c + 1) ? cmk(1.0, 0.0) : cmul(xbuf[i], scale);
         vy += v.x * y.x + v.y * y.y;
       }
       for (int o = 16; o > 0; o >>= 1) vy += __shfl_xor_sync(0xffffffffu, vy, o);
       if (lane < CL) cl.map_shared_rank(s_vav, lane)[rank] = vy;
     }
+    // v into vbuf and over column c of own packed rows (dead from here on): the
+    // reflectors go to C once, at the end, so no global store is pending at a
+    // cluster barrier
+    for (int i = c + 1 + tid; i < m; i += TT) {
+      const cplx v = (i == c + 1) ? cmk(1.0, 0.0) : cmul(xbuf[i], scale);
+      vbuf[i] = v;
+      if (i % CL == rank) stT(A + row_off<CL>(rank, i / CL) + c, v);  // unit entry explicit
+    }
     cl.sync();
     // ---- alpha = -|tau|^2/2 v^H C22 v (real; the panel kernel's form), the
-    //      same sum in every CTA; w = w0 + alpha v ------------------------------
-    double vav = 0.0;
-    for (int q = 0; q < CL; ++q) vav += s_vav[q];
-    const double alpha = -0.5 * (tau.x * tau.x + tau.y * tau.y) * vav;
-    for (int j = c + 1 + tid; j < m; j += TT) {
-      const cplx w = wbuf[j], v = vbuf[j];
-      wbuf[j] = cmk(w.x + alpha * v.x, w.y + alpha * v.y);
-    }
-    __syncthreads();
+    //      same sum in every CTA.  With w = w0 + alpha v,
+    //        v w^H + w v^H = v w0^H + (w0 + 2 alpha v) v^H,
+    //      so alpha goes into the factor of the row and w is never formed --------
+    double vv[4] = {};
+#pragma unroll
+    for (int q = 0; q < CL; ++q) vv[q & 3] += s_vav[q];
+    const double alpha2 = -(tau.x * tau.x + tau.y * tau.y) * ((vv[0] + vv[1]) + (vv[2] + vv[3]));  // 2 alpha
     // ---- C22 -= v w^H + w v^H on own rows; the updated column c + 1 goes out
     //      at once (x of the next column, d(c + 1)) ----------------------------
     for (int s = s_lo + warp; s < nslot; s += NW) {
       const int i = rank + CL * s;
       T2* row = A + row_off<CL>(rank, s);
-      const cplx vi = vbuf[i], wi = wbuf[i];
+      const cplx vi = vbuf[i], w0i = wbuf[i], wi = cmk(w0i.x + alpha2 * vi.x, w0i.y + alpha2 * vi.y);
       // v_i conj(w_j) + w_i conj(v_j) off the diagonal, two entries per step
       int j = c + 1 + lane;
       for (; j + 32 < i; j += 64) {
@@ -269,7 +273,7 @@ __global__ void __launch_bounds__(TT, 1) k_tridiag_tail(int n, int c0, T2* C, lo
       }
       if (lane == 0) {
         cplx a = ldT(row + i);
-        a.x -= 2.0 * (vi.x * wi.x + vi.y * wi.y);
+        a.x -= vi.x * (w0i.x + wi.x) + vi.y * (w0i.y + wi.y);
         a.y = 0.0;
         stT(row + i, a);
       }

@@ -1,21 +1,26 @@
 // Eigenpairs of the real symmetric tridiagonal T = tridiag(e, d, e).
 //
 // Eigenvalues (DSTEBZ, external/LAPACK/zheevx.f:490, range 'I'): one CTA of T
-// threads per requested eigenvalue index, multisection on the Sturm count (T
-// points per step, the interval shrinks T + 1 times) from the Gershgorin
+// threads per requested eigenvalue index, multisection on the Sturm count (2 T
+// points per step, the interval shrinks 2 T + 1 times) from the Gershgorin
 // interval; stop when the width is below max(abstol, pivmin,
 // 2 ulp max(|lo|,|hi|)) exactly as DSTEBZ's bisection test.
 //
 // Eigenvectors (DSTEIN, zheevx.f:496): inverse iteration with the shifted
 // tridiagonal factored by Gaussian elimination with partial pivoting, at
 // most five iterations, growth test sqrt(0.1/n) plus two extra iterations,
-// unit 2-norm with the largest component positive.  Eigenvalues closer than
+// unit 2-norm with the largest component positive; pivots below eps ||T|| become
+// that (a shift can meet an eigenvalue exactly beside couplings of 1e-170, whose
+// reciprocals as pivots overflowed the vector).  Eigenvalues closer than
 // CLUSTER_REL * ||T|| form a cluster: its shifts are separated by 10 ulp
 // (DSTEIN's perturbation) and its vectors are Gram-Schmidt orthogonalised
 // against the earlier members inside the iteration.  Residual loss of
 // orthogonality between well-separated vectors is removed afterwards by a
 // Cholesky-QR pass on the complex vectors (see solve.cu).
 #include "handle.cuh"
+
+#include <algorithm>
+#include <cmath>
 
 namespace {
 
@@ -31,27 +36,110 @@ __device__ __forceinline__ double recip_nr(double q) {
   return r;
 }
 
-// Number of eigenvalues of T below x (Sturm sequence of the LDL^T pivots).
-// The pivot recurrence q_i = d_i - x - e_{i-1}^2 / q_{i-1} uses recip_nr
-// instead of a division: within an ulp or so of the quotient, i.e. a relative
-// perturbation of e^2 of the order of the rounding the count already carries
-// (the count stays that of a nearby tridiagonal matrix), on a dependent chain
-// much shorter than a correctly rounded division.
-__device__ __forceinline__ int sturm_count(int n, const double* __restrict__ d,
-                                           const double* __restrict__ e2, double x, double pivmin) {
-  double q = d[0] - x;
-  if (fabs(q) <= pivmin) q = -pivmin;
-  int cnt = q < 0.0;
-  for (int i = 1; i < n; ++i) {
-    q = fma(-e2[i - 1], recip_nr(q), d[i] - x);
+// Sturm counts: the numbers of eigenvalues of T below the points x[0..NPT), from
+// the signs of the pivots q_i = d_i - x - e_{i-1}^2 / q_{i-1} of T - x, with
+// |q_i| <= pivmin replaced by -pivmin (DSTEBZ).  de[i] = (d_i, e_{i-1}^2).
+//
+// As quotients a step is a reciprocal and a product, 82 clocks one after the
+// other.  The leading minors p_i = q_i p_{i-1} follow
+//   p_i = (d_i - x) p_{i-1} - e_{i-1}^2 p_{i-2}
+// with one multiply-add on the chain (8 clocks), and q_i < 0 is a change of sign.
+// Each of the three roundings of a step is, as in the quotient form, a relative
+// change of d_i - x or e_{i-1}^2 of the order of an ulp: the count stays that of a
+// nearby tridiagonal matrix.  CH steps at a time run like this, from a pair scaled
+// by a power of two (exact) to order 1.  With ||T|| < 2^38 they grow by less than
+// 2^670, so nothing overflows, and a pair that had underflowed would still be below
+// 2^-250 at the end: then (and where ||T|| is larger, or a number is not finite) the
+// CH steps are done again as quotients.  What is left per step and point is three
+// operations of the double-precision pipe and one for the sign: two points per
+// thread share the loads, which run half of CH ahead.  k = 200, n = 1964:
+// 805 -> 411 us; k = 20, n = 316: 120 -> 69 us (643 and 106 with the range of
+// every minor tested).
+constexpr int CH = 16;
+constexpr int HCH = CH / 2;
+constexpr int NPT = 2;
+
+// the m steps at de as quotients, from the pair (cur, prev)
+__device__ __noinline__ int sturm_quotients(int m, const double2* __restrict__ de, double x, double pivmin,
+                                            double& cur, double& prev) {
+  double q = cur / prev;
+  int cnt = 0;
+  if (fabs(q) <= pivmin) {  // counted by its sign so far
+    cnt = !signbit(q);
+    q = -pivmin;
+  }
+  for (int i = 0; i < m; ++i) {
+    const double2 t = de[i];
+    q = fma(-t.y, recip_nr(q), t.x - x);
     if (fabs(q) <= pivmin) q = -pivmin;
     cnt += q < 0.0;
   }
+  cur = q;
+  prev = 1.0;
   return cnt;
 }
 
-// scal[0] = gl, [1] = gu, [2] = pivmin, [3] = tnorm; e2[i] = e[i]^2
-__global__ void k_tridiag_prep(int n, const double* d, const double* e, double* e2, double* scal) {
+__device__ __forceinline__ int hiword(double v) { return __double2hiint(v) & 0x7fffffff; }
+
+// minors: ||T|| < 2^38
+__device__ __forceinline__ void sturm_count(int n, const double2* __restrict__ de, const double (&x)[NPT],
+                                            double pivmin, bool minors, int (&cnt)[NPT]) {
+  double cur[NPT], prev[NPT];
+#pragma unroll
+  for (int r = 0; r < NPT; ++r) {
+    cur[r] = de[0].x - x[r];
+    if (fabs(cur[r]) <= pivmin) cur[r] = -pivmin;
+    prev[r] = 1.0;
+    cnt[r] = cur[r] < 0.0;
+  }
+  int i = 1;
+  if (minors) {
+    double2 t[2][HCH];
+#pragma unroll
+    for (int u = 0; u < HCH; ++u) t[0][u] = de[min(i + u, n - 1)];
+    for (; i + CH <= n; i += CH) {
+      double c0[NPT], p0[NPT];
+      unsigned sg[NPT];
+#pragma unroll
+      for (int r = 0; r < NPT; ++r) {
+        c0[r] = cur[r]; p0[r] = prev[r];
+        const int big = max(hiword(cur[r]), hiword(prev[r])) & 0x7ff00000;
+        const double sc = __hiloint2double(min(max(0x7fe00000 - big, 0x00100000), 0x7fe00000), 0);
+        cur[r] *= sc; prev[r] *= sc;
+        sg[r] = (unsigned)__double2hiint(cur[r]) >> 31;
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+#pragma unroll
+        for (int u = 0; u < HCH; ++u) t[h ^ 1][u] = de[min(i + (h + 1) * HCH + u, n - 1)];
+#pragma unroll
+        for (int u = 0; u < HCH; ++u)
+#pragma unroll
+          for (int r = 0; r < NPT; ++r) {
+            const double nx = fma(t[h][u].x - x[r], cur[r], -(t[h][u].y * prev[r]));
+            sg[r] = __funnelshift_l((unsigned)__double2hiint(nx), sg[r], 1);  // the sign bits, newest last
+            prev[r] = cur[r];
+            cur[r] = nx;
+          }
+      }
+#pragma unroll
+      for (int r = 0; r < NPT; ++r) {
+        const int big = max(hiword(cur[r]), hiword(prev[r]));
+        if (big > 0x3ff00000 - (250 << 20) && big < 0x7ff00000) {
+          cnt[r] += __popc((sg[r] ^ (sg[r] >> 1)) & ((1u << CH) - 1u));
+        } else {
+          cur[r] = c0[r]; prev[r] = p0[r];
+          cnt[r] += sturm_quotients(CH, de + i, x[r], pivmin, cur[r], prev[r]);
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < NPT; ++r) cnt[r] += sturm_quotients(n - i, de + i, x[r], pivmin, cur[r], prev[r]);
+}
+
+// scal[0] = gl, [1] = gu, [2] = pivmin, [3] = tnorm; de[i] = (d[i], e[i-1]^2)
+__global__ void k_tridiag_prep(int n, const double* d, const double* e, double2* de, double* scal) {
   __shared__ double s_lo[256], s_hi[256], s_e2[256], s_nrm[256];
   double lo = 1e300, hi = -1e300, em = 0.0, nm = 0.0;
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
@@ -60,10 +148,9 @@ __global__ void k_tridiag_prep(int n, const double* d, const double* e, double* 
     lo = fmin(lo, d[i] - ea - eb);
     hi = fmax(hi, d[i] + ea + eb);
     nm = fmax(nm, fabs(d[i]) + ea + eb);
-    if (i < n - 1) {
-      e2[i] = e[i] * e[i];
-      em = fmax(em, e[i] * e[i]);
-    }
+    const double e2 = (i > 0) ? e[i - 1] * e[i - 1] : 0.0;
+    de[i] = make_double2(d[i], e2);
+    em = fmax(em, e2);
   }
   s_lo[threadIdx.x] = lo; s_hi[threadIdx.x] = hi; s_e2[threadIdx.x] = em; s_nrm[threadIdx.x] = nm;
   __syncthreads();
@@ -89,31 +176,41 @@ __global__ void k_tridiag_prep(int n, const double* d, const double* e, double* 
   }
 }
 
-// One CTA per eigenvalue index; all its threads are the points of a step.
-__global__ void k_stebz(int n, const double* d, const double* e2, const double* scal, int k,
-                        double abstol, double* w, int* status) {
+// One CTA per eigenvalue index; its threads' points (tid and tid + T) are a step's.
+__global__ void k_stebz(int n, const double2* de, const double* scal, int k, double abstol, double* w,
+                        int* status) {
   __shared__ int s_first[2][32];
   const int j = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, T = blockDim.x;
   const double pivmin = scal[2];
   const double ulp = 2.220446049250313e-16;
   const double atol = abstol > 0.0 ? abstol : ulp * scal[3];
+  const bool minors = scal[3] < 0x1p38;
   double lo = scal[0], hi = scal[1];
   bool conv = false;
   for (int it = 0; it < 200; ++it) {
     const double width = hi - lo;
     const double tol = fmax(fmax(atol, pivmin), 2.0 * ulp * fmax(fabs(lo), fabs(hi)));
     if (width <= tol) { conv = true; break; }
-    const double step = width / (T + 1);
-    const int cnt = sturm_count(n, d, e2, fmin(lo + (tid + 1) * step, hi), pivmin);
-    // the first point with at least j + 1 eigenvalues below it (T: none)
-    const unsigned ball = __ballot_sync(0xffffffffu, cnt >= j + 1);
-    if (lane == 0) s_first[it & 1][warp] = ball ? 32 * warp + __ffs(ball) - 1 : T;
+    const double step = width / (NPT * T + 1);
+    double x[NPT];
+    int cnt[NPT];
+#pragma unroll
+    for (int r = 0; r < NPT; ++r) x[r] = fmin(lo + (tid + r * T + 1) * step, hi);
+    sturm_count(n, de, x, pivmin, minors, cnt);
+    // the first point with at least j + 1 eigenvalues below it (NPT T: none)
+    int mine = NPT * T;
+#pragma unroll
+    for (int r = NPT - 1; r >= 0; --r) {
+      const unsigned ball = __ballot_sync(0xffffffffu, cnt[r] >= j + 1);
+      if (ball) mine = r * T + 32 * warp + __ffs(ball) - 1;
+    }
+    if (lane == 0) s_first[it & 1][warp] = mine;
     __syncthreads();
-    int f = T;
+    int f = NPT * T;
     for (int q = 0; q < T / 32; ++q) f = min(f, s_first[it & 1][q]);
     const double l0 = lo;
     if (f > 0) lo = fmin(l0 + f * step, hi);
-    if (f < T) hi = fmin(l0 + (f + 1) * step, hi);
+    if (f < NPT * T) hi = fmin(l0 + (f + 1) * step, hi);
     if (!(hi > lo)) { conv = true; break; }
   }
   if (tid == 0) {
@@ -181,7 +278,7 @@ __global__ void k_stein(int n, const double* __restrict__ d, const double* __res
         a = dd - m * b;
         b = ee;
       } else {
-        const double rc = 1.0 / c;
+        const double rc = 1.0 / ((fabs(c) < pert) ? copysign(pert, c) : c);
         ua[o] = rc; ub[o] = dd; uf[o] = ee;
         const double m = a * rc;
         um[o] = -m - 2.0;  // encodes a swap (a multiplier |m| <= 1 never reaches below -1)
@@ -272,7 +369,11 @@ __global__ void k_stein(int n, const double* __restrict__ d, const double* __res
 // runs the recurrences (factorisation, forward elimination, back
 // substitution) at shared-memory latency, the warp shares the element-wise
 // passes.  The finished vectors go to Yi (interleaved as in k_stein) because
-// later members of a cluster are orthogonalised against them.
+// later members of a cluster are orthogonalised against them.  The recurrences
+// are what it takes its time for: SCH rows at a time are loaded before any of them
+// is stored (a load does not pass a store that may alias it) and swaps are
+// selections.  k = 200, n = 1964: 639 -> 394 us; k = 20, n = 316: 108 -> 69 us.
+constexpr int SCH = 8;
 __global__ void __launch_bounds__(32) k_stein_smem(int n, const double* __restrict__ d,
                                                    const double* __restrict__ e,
                                                    const double* __restrict__ scal, int k,
@@ -305,25 +406,28 @@ __global__ void __launch_bounds__(32) k_stein_smem(int n, const double* __restri
     __shared__ double s_ulast;
     if (lane == 0) {
       double a = d[0] - lam, b = (n > 1) ? e[0] : 0.0;
-      for (int i = 0; i < n - 1; ++i) {
-        const double c = e[i], dd = d[i + 1] - lam, ee = (i + 1 < n - 1) ? e[i + 1] : 0.0;
-        if (fabs(a) >= fabs(c)) {
-          const double aa = (fabs(a) < pert) ? copysign(pert, a) : a;
-          const double r = 1.0 / aa;
-          ra[i] = r; rb[i] = b; rf[i] = 0.0;
-          const double m = c * r;
-          rm[i] = m;
-          a = dd - m * b;
-          b = ee;
-        } else {
-          const double r = 1.0 / c;
-          ra[i] = r; rb[i] = dd; rf[i] = ee;
-          const double m = a * r;
-          rm[i] = -m - 2.0;
-          a = b - m * dd;
-          b = -m * ee;
-        }
+      auto row = [&](int i, double c, double dd, double ee) {
+        const bool sw = !(fabs(a) >= fabs(c));
+        double piv = sw ? c : a;
+        if (fabs(piv) < pert) piv = copysign(pert, piv);
+        const double r = 1.0 / piv, m = (sw ? a : c) * r;
+        ra[i] = r;
+        rb[i] = sw ? dd : b;
+        rf[i] = sw ? ee : 0.0;
+        rm[i] = sw ? -m - 2.0 : m;
+        a = (sw ? b : dd) - m * (sw ? dd : b);
+        b = sw ? -m * ee : ee;
+      };
+      int i = 0;
+      for (; i + SCH < n - 1; i += SCH) {
+        double ev[SCH + 1], dv[SCH];
+#pragma unroll
+        for (int u = 0; u < SCH; ++u) { ev[u] = e[i + u]; dv[u] = d[i + u + 1] - lam; }
+        ev[SCH] = e[i + SCH];
+#pragma unroll
+        for (int u = 0; u < SCH; ++u) row(i + u, ev[u], dv[u], ev[u + 1]);
       }
+      for (; i < n - 1; ++i) row(i, e[i], d[i + 1] - lam, (i + 1 < n - 1) ? e[i + 1] : 0.0);
       const double aa = (fabs(a) < pert) ? copysign(pert, a) : a;
       ra[n - 1] = 1.0 / aa;
       rb[n - 1] = 0.0; rf[n - 1] = 0.0; rm[n - 1] = 0.0;
@@ -340,26 +444,45 @@ __global__ void __launch_bounds__(32) k_stein_smem(int n, const double* __restri
       for (int o = 16; o > 0; o >>= 1) s1 += __shfl_xor_sync(0xffffffffu, s1, o);
       const double scl = (s1 > 0.0) ? n * tnorm * fmax(eps, ulast) / s1 : 1.0;
       if (lane == 0) {
+        // forward elimination; a swapped row keeps the next entry and goes on with
+        // cur + (m + 2) next, the others keep cur and go on with next - m cur
         double cur = y[0] * scl;
-        for (int i = 0; i < n - 1; ++i) {
-          const double nx = y[i + 1] * scl;
-          const double m = rm[i];
-          if (m < -1.0) {
-            y[i] = nx;
-            cur = cur + (m + 2.0) * nx;
-          } else {
-            y[i] = cur;
-            cur = nx - m * cur;
-          }
+        auto fwd = [&](double m, double nx) {
+          const bool sw = m < -1.0;
+          const double kept = sw ? nx : cur;
+          cur = fma(sw ? m + 2.0 : -m, kept, sw ? cur : nx);
+          return kept;
+        };
+        int i = 0;
+        for (; i + SCH <= n - 1; i += SCH) {
+          double mv[SCH], yv[SCH];
+#pragma unroll
+          for (int u = 0; u < SCH; ++u) { mv[u] = rm[i + u]; yv[u] = y[i + u + 1] * scl; }
+#pragma unroll
+          for (int u = 0; u < SCH; ++u) y[i + u] = fwd(mv[u], yv[u]);
         }
+        for (; i < n - 1; ++i) y[i] = fwd(rm[i], y[i + 1] * scl);
+        // back substitution: the reciprocal pivot goes into the factors first, so a
+        // row adds one multiply-add to the chain
         double x2 = 0.0, x1 = cur * ra[n - 1];
         y[n - 1] = x1;
-        for (int i = n - 2; i >= 0; --i) {
-          const double x = (y[i] - rb[i] * x1 - rf[i] * x2) * ra[i];
-          y[i] = x;
+        auto bwd = [&](double p, double b, double f, double c) {
+          const double x = fma(-(b * p), x1, fma(-(f * p), x2, c * p));
           x2 = x1;
           x1 = x;
+          return x;
+        };
+        i = n - 2;
+        for (; i - SCH + 1 >= 0; i -= SCH) {
+          double pv[SCH], bv[SCH], fv[SCH], yv[SCH];
+#pragma unroll
+          for (int u = 0; u < SCH; ++u) {
+            pv[u] = ra[i - u]; bv[u] = rb[i - u]; fv[u] = rf[i - u]; yv[u] = y[i - u];
+          }
+#pragma unroll
+          for (int u = 0; u < SCH; ++u) y[i - u] = bwd(pv[u], bv[u], fv[u], yv[u]);
         }
+        for (; i >= 0; --i) y[i] = bwd(ra[i], rb[i], rf[i], y[i]);
       }
       __syncwarp();
       for (int q = j0; q < j; ++q) {
@@ -414,27 +537,33 @@ __global__ void k_y_to_z(int n, int k, const double* Yi, cplx* Z, long long ldz)
 }  // namespace
 
 // Lowest k eigenvalues into w, eigenvectors as complex columns of Z (n x k).
-// scratch: e2 (n), scal (4), cl (k ints), 4*n*k doubles for the factors, n*k for Yi.
+// scratch: de (2n), scal (8), 4*n*k doubles for the factors, n*k for Yi; 16-byte aligned.
 int tridiag_eig(excfv_handle* h, int n, int k, double abstol, const double* d, const double* e,
                 double* w, cplx* Z, long long ldz, double* scratch, int* iscratch) {
   cudaStream_t s = h->stream;
-  double* e2 = scratch;
-  double* scal = scratch + n;
+  double2* de = reinterpret_cast<double2*>(scratch);
+  double* scal = scratch + 2 * (size_t)n;
   double* ua = scal + 8;
   double* ub = ua + (size_t)n * k;
   double* uf = ub + (size_t)n * k;
   double* um = uf + (size_t)n * k;
   double* Yi = um + (size_t)n * k;
-  k_tridiag_prep<<<1, 256, 0, s>>>(n, d, e, e2, scal); count_launch();
+  k_tridiag_prep<<<1, 256, 0, s>>>(n, d, e, de, scal); count_launch();
   CUDA_TRY(cudaGetLastError());
-  // A step costs a Sturm chain of n dependent steps (82 clocks each) however many
-  // points it has, until the reciprocals fill their unit at about 8 warps per SM
-  // of the handle's budget: as many points as that allows (k = 20: 256 points and
-  // 7 steps instead of 32 and 10; 1024 points took 215 us where 32 took 160).
+  // Threads per eigenvalue: a pass narrows the interval 2 T + 1 times and takes n
+  // times the larger of one warp's latency, about 22 clocks, and 16 issue slots per
+  // warp of an SM quarter (two points of three double-precision operations of two
+  // slots each, signs and loads); the T with the shortest product of passes (for 50
+  // bits) and step.
   const int sms = (h->grid_ctas > 0) ? h->grid_ctas : h->nsm;
   int T = 32;
-  while (T < 256 && (long long)2 * T * k <= 256LL * sms) T *= 2;
-  k_stebz<<<k, T, 0, s>>>(n, d, e2, scal, k, abstol, w, h->ws.status); count_launch();
+  double best = 1e300;
+  for (int t = 32; t <= 256; t *= 2) {
+    const double warps = (double)((k + sms - 1) / sms) * t / 128.0;
+    const double est = std::ceil(50.0 / std::log2(NPT * t + 1.0)) * std::max(22.0, 16.0 * warps);
+    if (est < best) { best = est; T = t; }
+  }
+  k_stebz<<<k, T, 0, s>>>(n, de, scal, k, abstol, w, h->ws.status); count_launch();
   CUDA_TRY(cudaGetLastError());
   k_clusters<<<(k + 127) / 128, 128, 0, s>>>(k, w, scal, iscratch); count_launch();
   CUDA_TRY(cudaGetLastError());
@@ -452,4 +581,4 @@ int tridiag_eig(excfv_handle* h, int n, int k, double abstol, const double* d, c
   return EXCFV_OK;
 }
 
-size_t tridiag_eig_scratch_doubles(int n, int k) { return (size_t)n + 8 + 5 * (size_t)n * k; }
+size_t tridiag_eig_scratch_doubles(int n, int k) { return 2 * (size_t)n + 8 + 5 * (size_t)n * k; }

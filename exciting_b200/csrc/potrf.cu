@@ -19,16 +19,18 @@ constexpr int NBP = 64;
 // One CTA factors the b x b diagonal block (b <= 64) and inverts the factor: a
 // right-looking elimination of [A | I] in steps of four columns, which leaves
 // U = L^H in A and L^-1 = (U^-1)^H in the unit part.  Per step
-//   the two warps that own the 64 active columns (A's columns right of the
-//   step, the unit part's up to it) each factor the 4 x 4 diagonal block
-//   redundantly in registers and solve their own column's four entries;
+//   the two pivot warps, a thread per active column (A's columns right of the step,
+//   the unit part's up to it), each factor the 4 x 4 diagonal block redundantly in
+//   registers and solve their own column's four entries;
 //   --- barrier ---
-//   every warp updates four rows at a time with the four pivot rows;
-//   --- barrier ---
-// so 16 steps cost 32 barriers and a chain of four rsqrt each.  Bound by that
-// chain and by shared-memory traffic (four rows share each pivot-row load).
-// A 64-block takes 30 us and a 22-block 15; a column at a time with 1024 threads
-// and ~260 barriers took 57 us for either.
+//   the pivot warps update the four rows of the next step, each thread its own
+//   column, and go on to the next diagonal block at once (a barrier of their own);
+//   beside them the other 14 warps update the rows below, four rows at a time with
+//   the four pivot rows
+// so a step has one block barrier and takes the longer of the pivots' chain (four
+// reciprocal square roots) and the update.  A 64-block takes 24 us and a 22-block
+// 13; with all warps updating between two barriers it was 30 and 15, a column at a
+// time with 1024 threads and ~260 barriers 57 us for either.
 constexpr int LDB = 65;
 constexpr int DT = 512;
 
@@ -44,7 +46,7 @@ __device__ __forceinline__ int chol4(const cplx* A, int j, cplx (&u)[4][4], doub
   for (int k = 0; k < 4; ++k) {
     const double d = u[k][k].x;
     if (!(d > 0.0)) return k + 1;
-    r[k] = 1.0 / sqrt(d);
+    r[k] = rsqrt(d);
 #pragma unroll
     for (int c = k; c < 4; ++c) u[k][c] = (c == k) ? cmk(d * r[k], 0.0) : cscale(u[k][c], r[k]);
 #pragma unroll
@@ -59,7 +61,7 @@ __device__ __forceinline__ void potrf_diag_block(int n, int kb, cplx* O, long lo
   extern __shared__ __align__(16) unsigned char dsm[];
   cplx* A = reinterpret_cast<cplx*>(dsm);   // 64 x LDB, row-major [r][c]
   cplx* Y = A + NBP * LDB;                  // the unit part, L^-1 at the end
-  __shared__ int s_fail;
+  __shared__ int s_fail[2];  // by the parity of the step: the pivot warps run ahead
   if (status[ST_POTRF] != 0) return;
   const int b = min(NBP, n - kb);
   const int lim = (b + 3) / 4 * 4;          // rows past b are padded with the identity
@@ -72,20 +74,20 @@ __device__ __forceinline__ void potrf_diag_block(int n, int kb, cplx* O, long lo
     if (r == c) a.y = 0.0;
     A[r * LDB + c] = a;
   }
-  if (tid == 0) s_fail = 0;
+  if (tid < 2) s_fail[tid] = 0;
   __syncthreads();
   for (int j = 0; j < lim; j += 4) {
-    cplx u[4][4];
+    int& fail = s_fail[(j >> 2) & 1];
+    cplx u[4][4], x[4];
     double r[4];
+    // columns right of the step in A, then columns 0 .. j + 3 of the unit part
+    const bool mineA = tid < 60 - j;
+    cplx* col = mineA ? A + j + 4 + tid : Y + tid - (60 - j);
     if (tid < 64) {
       const int bad = chol4(A, j, u, r);
       if (bad) {
-        if (tid == 0) s_fail = j + bad;
+        if (tid == 0) fail = j + bad;
       } else {
-        // columns right of the step in A, then columns 0 .. j + 3 of the unit part
-        const bool inA = tid < 60 - j;
-        cplx* col = inA ? A + j + 4 + tid : Y + tid - (60 - j);
-        cplx x[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
           x[k] = col[(j + k) * LDB];
@@ -96,42 +98,56 @@ __device__ __forceinline__ void potrf_diag_block(int n, int kb, cplx* O, long lo
         }
       }
     }
-    __syncthreads();
-    if (s_fail) {
-      if (tid == 0 && s_fail <= b) atomicCAS(&status[ST_POTRF], 0, kb + s_fail);
+    __syncthreads();  // the pivot rows are there, the rows from j + 4 on have the last step's update
+    if (fail) {
+      if (tid == 0 && fail <= b) atomicCAS(&status[ST_POTRF], 0, kb + fail);
       return;
     }
-    if (tid == 0) {
+    // rows i of both parts: row -= sum_k conj(U(j+k, i)) (row j+k)
+    if (tid < 64) {
+      if (tid == 0) {
 #pragma unroll
-      for (int k = 0; k < 4; ++k)
+        for (int k = 0; k < 4; ++k)
 #pragma unroll
-        for (int c = k; c < 4; ++c) A[(j + k) * LDB + j + c] = u[k][c];
-    }
-    // rows i = j + 4 + warp + 16 q of both parts: row -= sum_k conj(U(j+k, i)) (row j+k)
-    const int i0 = j + 4 + warp;
-    if (i0 < lim) {
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int c = lane + 32 * h;
-        const bool inA = c >= j + 4;
-        cplx* M = inA ? A : Y;
-        if (c >= lim) continue;
-        cplx pv[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) pv[k] = M[(j + k) * LDB + c];
+          for (int c = k; c < 4; ++c) A[(j + k) * LDB + j + c] = u[k][c];
+      }
+      if (j + 4 < lim) {
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-          const int i = i0 + 16 * q;
-          if (i >= lim || (inA && c < i)) continue;
-          cplx v = M[i * LDB + c];
+          const int i = j + 4 + q;
+          cplx v = col[i * LDB];
 #pragma unroll
-          for (int k = 0; k < 4; ++k) v = csub(v, cmulc(A[(j + k) * LDB + i], pv[k]));
-          M[i * LDB + c] = v;
+          for (int k = 0; k < 4; ++k) v = csub(v, cmulc(A[(j + k) * LDB + i], x[k]));
+          col[i * LDB] = v;
+        }
+      }
+      asm volatile("bar.sync 1, 64;" ::: "memory");
+    } else {
+      const int i0 = j + 6 + warp;
+      if (i0 < lim) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int c = lane + 32 * h;
+          const bool inA = c >= j + 4;
+          cplx* M = inA ? A : Y;
+          if (c >= lim) continue;
+          cplx pv[4];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) pv[k] = M[(j + k) * LDB + c];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const int i = i0 + 14 * q;
+            if (i >= lim || (inA && c < i)) continue;
+            cplx v = M[i * LDB + c];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) v = csub(v, cmulc(A[(j + k) * LDB + i], pv[k]));
+            M[i * LDB + c] = v;
+          }
         }
       }
     }
-    __syncthreads();
   }
+  __syncthreads();
   for (int t = tid; t < NBP * NBP; t += DT) {
     const int r = t % NBP, c = t / NBP;
     if (r < b && c < b && r <= c) {

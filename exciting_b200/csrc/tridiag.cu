@@ -828,9 +828,9 @@ int tridiag_tail(excfv_handle* h, int n, int c0, T2* C, long long ld);
 // the last columns (tridiag_tail.cu): as soon as the cluster holds the block
 // where the barrier kernel reduces the panels; where the dataflow kernel does
 // (G blocks), once the block is so small that the cluster is faster.  The
-// cluster takes 4.4 us per column below m = 200, 6.2 up to 316 and 9.2 from
-// there to 608, the dataflow panels about 6.5 with their share of the updates:
-// order 484 takes 4.76, 4.65 and 4.82 ms with the tail from 192, 320 and 448.
+// cluster takes 4.1 us per column over the last 300 and more above, the dataflow
+// panels about 6 with their share of the updates: order 484 takes 3.85, 3.90 and
+// 4.00 ms with the tail from 320, 384 and 448, order 715 6.17, 6.22 and 6.33.
 constexpr int FLOW_TAIL = 320;
 static int tail_start(int n, bool complex64, int G) {
   int tail_max = complex64 ? tridiag_tail_max<float2>() : tridiag_tail_max<double2>();

@@ -564,9 +564,9 @@ def main():
     hbm = peaks.get("hbm_gbs") or 6650.0
     hbm_src = "measured" if peaks.get("hbm_gbs") else "fallback"
     if p_ms >= g_ms:
-        roof = {"kernel": "k_tridiag_panel", "bound": "hbm", "achieved": p_ach, "peak": hbm,
+        roof = {"kernel": "k_tridiag_flow", "bound": "hbm", "achieved": p_ach, "peak": hbm,
                 "unit": "GB/s", "frac": (p_ach / hbm) if p_ach else None,
-                "traffic": traffic.get("k_tridiag_panel"),
+                "traffic": traffic.get("k_tridiag_flow"),
                 "algorithmic": "16*m(m+1)/2 bytes (lower triangle of the m x m trailing block, y = C22 v) per reduced column, summed over the launch's columns",
                 "panel_columns": c_tail, "tail_columns": n - 1 - c_tail,
                 "peak_source": f"{hbm_src} HBM copy (MEASURED_PEAKS.json)"}

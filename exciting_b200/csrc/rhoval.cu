@@ -453,26 +453,31 @@ int stage_set_rho(excfv_handle* h, const excfv_rhoset* r) {
   d.nrcmax = (nrmax + r->lradstep - 1) / r->lradstep;
   const int nlomax = std::max(st.nlomax, 1);
   const int L1 = r->lmaxvr + 1;
-  // radial functions on the coarse mesh (function values only)
+  std::vector<int> first(st.natmtot, -1);
+  for (int a = 0; a < st.natmtot && a < (int)st.h_lo_first.size(); ++a) first[a] = st.h_lo_first[a];
+  // Radial functions on the coarse mesh (function values only).  k_rho_psi sums
+  // over every slot of an atom, so the slots that its species does not have (and
+  // orbitals above lmaxvr) are zeros here: the caller's arrays may hold anything
+  // there, and a NaN times the slot's zero coefficient would be a NaN.
   std::vector<double> u((size_t)d.nrcmax * st.apwordmax * L1 * st.natmtot, 0.0);
   std::vector<double> v((size_t)d.nrcmax * nlomax * st.natmtot, 0.0);
   for (int ias = 0; ias < st.natmtot; ++ias) {
     const int is = st.h_idxis[ias];
     const int nrc = (r->nrmt[is] + r->lradstep - 1) / r->lradstep;
-    for (int irc = 0; irc < nrc; ++irc) {
-      const size_t ir = (size_t)irc * r->lradstep;
-      for (int l = 0; l < L1; ++l)
-        for (int io = 0; io < st.apwordmax; ++io)
-          u[irc + (size_t)d.nrcmax * (io + (size_t)st.apwordmax * (l + (size_t)L1 * ias))] =
-              r->apwfr[ir + (size_t)r->nrmtmax * (2 * (io + (size_t)st.apwordmax * (l + (size_t)(st.lmaxapw + 1) * ias)))];
-      if (r->lofr)
-        for (int ilo = 0; ilo < st.nlomax; ++ilo)
-          v[irc + (size_t)d.nrcmax * (ilo + (size_t)nlomax * ias)] =
-              r->lofr[ir + (size_t)r->nrmtmax * (2 * (ilo + (size_t)nlomax * ias))];
+    for (int l = 0; l < L1; ++l)
+      for (int io = 0; io < st.h_apword[l + (size_t)(st.lmaxapw + 1) * is]; ++io) {
+        double* dst = &u[(size_t)d.nrcmax * (io + (size_t)st.apwordmax * (l + (size_t)L1 * ias))];
+        const double* src =
+            r->apwfr + (size_t)r->nrmtmax * (2 * (io + (size_t)st.apwordmax * (l + (size_t)(st.lmaxapw + 1) * ias)));
+        for (int irc = 0; irc < nrc; ++irc) dst[irc] = src[(size_t)irc * r->lradstep];
+      }
+    for (int ilo = 0; st.nlotot > 0 && ilo < std::min(st.h_nlorb[is], st.nlomax); ++ilo) {
+      if (st.h_lorbl[ilo + (size_t)nlomax * is] > r->lmaxvr) continue;
+      double* dst = &v[(size_t)d.nrcmax * (ilo + (size_t)nlomax * ias)];
+      const double* src = r->lofr + (size_t)r->nrmtmax * (2 * (ilo + (size_t)nlomax * ias));
+      for (int irc = 0; irc < nrc; ++irc) dst[irc] = src[(size_t)irc * r->lradstep];
     }
   }
-  std::vector<int> first(st.natmtot, -1);
-  for (int a = 0; a < st.natmtot && a < (int)st.h_lo_first.size(); ++a) first[a] = st.h_lo_first[a];
   const size_t L = d.lmmaxvr;
   d.ncoef = (size_t)st.apwordmax * L * std::max(st.nstfv, 1) * st.natmtot;
   d.gang_elems = rho_gang_elems((size_t)2 * std::max(st.nstfv, 1), L1 * st.apwordmax + nlomax, L, st.natmtot);

@@ -18,6 +18,7 @@
 // orthogonality between well-separated vectors is removed afterwards by a
 // Cholesky-QR pass on the complex vectors (see solve.cu).
 #include "handle.cuh"
+#include "sturm.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -25,118 +26,6 @@
 namespace {
 
 constexpr double CLUSTER_REL = 1e-9;
-
-// 1/q from the hardware approximation refined by two Newton-Raphson steps
-// r <- r (2 - q r) (each roughly doubles the correct bits).
-__device__ __forceinline__ double recip_nr(double q) {
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(q));
-  r = fma(r, fma(-q, r, 1.0), r);
-  r = fma(r, fma(-q, r, 1.0), r);
-  return r;
-}
-
-// Sturm counts: the numbers of eigenvalues of T below the points x[0..NPT), from
-// the signs of the pivots q_i = d_i - x - e_{i-1}^2 / q_{i-1} of T - x, with
-// |q_i| <= pivmin replaced by -pivmin (DSTEBZ).  de[i] = (d_i, e_{i-1}^2).
-//
-// As quotients a step is a reciprocal and a product, 82 clocks one after the
-// other.  The leading minors p_i = q_i p_{i-1} follow
-//   p_i = (d_i - x) p_{i-1} - e_{i-1}^2 p_{i-2}
-// with one multiply-add on the chain (8 clocks), and q_i < 0 is a change of sign.
-// Each of the three roundings of a step is, as in the quotient form, a relative
-// change of d_i - x or e_{i-1}^2 of the order of an ulp: the count stays that of a
-// nearby tridiagonal matrix.  CH steps at a time run like this, from a pair scaled
-// by a power of two (exact) to order 1.  With ||T|| < 2^38 they grow by less than
-// 2^670, so nothing overflows, and a pair that had underflowed would still be below
-// 2^-250 at the end: then (and where ||T|| is larger, or a number is not finite) the
-// CH steps are done again as quotients.  What is left per step and point is three
-// operations of the double-precision pipe and one for the sign: two points per
-// thread share the loads, which run half of CH ahead.  k = 200, n = 1964:
-// 805 -> 411 us; k = 20, n = 316: 120 -> 69 us (643 and 106 with the range of
-// every minor tested).
-constexpr int CH = 16;
-constexpr int HCH = CH / 2;
-constexpr int NPT = 2;
-
-// the m steps at de as quotients, from the pair (cur, prev)
-__device__ __noinline__ int sturm_quotients(int m, const double2* __restrict__ de, double x, double pivmin,
-                                            double& cur, double& prev) {
-  double q = cur / prev;
-  int cnt = 0;
-  if (fabs(q) <= pivmin) {  // counted by its sign so far
-    cnt = !signbit(q);
-    q = -pivmin;
-  }
-  for (int i = 0; i < m; ++i) {
-    const double2 t = de[i];
-    q = fma(-t.y, recip_nr(q), t.x - x);
-    if (fabs(q) <= pivmin) q = -pivmin;
-    cnt += q < 0.0;
-  }
-  cur = q;
-  prev = 1.0;
-  return cnt;
-}
-
-__device__ __forceinline__ int hiword(double v) { return __double2hiint(v) & 0x7fffffff; }
-
-// minors: ||T|| < 2^38
-__device__ __forceinline__ void sturm_count(int n, const double2* __restrict__ de, const double (&x)[NPT],
-                                            double pivmin, bool minors, int (&cnt)[NPT]) {
-  double cur[NPT], prev[NPT];
-#pragma unroll
-  for (int r = 0; r < NPT; ++r) {
-    cur[r] = de[0].x - x[r];
-    if (fabs(cur[r]) <= pivmin) cur[r] = -pivmin;
-    prev[r] = 1.0;
-    cnt[r] = cur[r] < 0.0;
-  }
-  int i = 1;
-  if (minors) {
-    double2 t[2][HCH];
-#pragma unroll
-    for (int u = 0; u < HCH; ++u) t[0][u] = de[min(i + u, n - 1)];
-    for (; i + CH <= n; i += CH) {
-      double c0[NPT], p0[NPT];
-      unsigned sg[NPT];
-#pragma unroll
-      for (int r = 0; r < NPT; ++r) {
-        c0[r] = cur[r]; p0[r] = prev[r];
-        const int big = max(hiword(cur[r]), hiword(prev[r])) & 0x7ff00000;
-        const double sc = __hiloint2double(min(max(0x7fe00000 - big, 0x00100000), 0x7fe00000), 0);
-        cur[r] *= sc; prev[r] *= sc;
-        sg[r] = (unsigned)__double2hiint(cur[r]) >> 31;
-      }
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-#pragma unroll
-        for (int u = 0; u < HCH; ++u) t[h ^ 1][u] = de[min(i + (h + 1) * HCH + u, n - 1)];
-#pragma unroll
-        for (int u = 0; u < HCH; ++u)
-#pragma unroll
-          for (int r = 0; r < NPT; ++r) {
-            const double nx = fma(t[h][u].x - x[r], cur[r], -(t[h][u].y * prev[r]));
-            sg[r] = __funnelshift_l((unsigned)__double2hiint(nx), sg[r], 1);  // the sign bits, newest last
-            prev[r] = cur[r];
-            cur[r] = nx;
-          }
-      }
-#pragma unroll
-      for (int r = 0; r < NPT; ++r) {
-        const int big = max(hiword(cur[r]), hiword(prev[r]));
-        if (big > 0x3ff00000 - (250 << 20) && big < 0x7ff00000) {
-          cnt[r] += __popc((sg[r] ^ (sg[r] >> 1)) & ((1u << CH) - 1u));
-        } else {
-          cur[r] = c0[r]; prev[r] = p0[r];
-          cnt[r] += sturm_quotients(CH, de + i, x[r], pivmin, cur[r], prev[r]);
-        }
-      }
-    }
-  }
-#pragma unroll
-  for (int r = 0; r < NPT; ++r) cnt[r] += sturm_quotients(n - i, de + i, x[r], pivmin, cur[r], prev[r]);
-}
 
 // scal[0] = gl, [1] = gu, [2] = pivmin, [3] = tnorm; de[i] = (d[i], e[i-1]^2)
 __global__ void k_tridiag_prep(int n, const double* d, const double* e, double2* de, double* scal) {

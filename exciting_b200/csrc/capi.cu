@@ -347,6 +347,7 @@ int stage_reserve(excfv_handle* h, int nmatmax, int ngkmax, int kmax) {
   kmax = std::max(kmax, ws.kmax);
   cudaStreamSynchronize(h->stream);
   free_workspace(ws);
+  h->ws_gen++;
   const DevStatic& st = h->st;
   const size_t n = nmatmax, n2 = n * n, AM = (size_t)st.natmtot * st.maxaa;
   const size_t K = kmax;
@@ -1609,7 +1610,10 @@ static std::vector<unsigned long long> batch_key(const excfv_handle* h, const Ba
                                        (unsigned long long)h->batch_form,
                                        (unsigned long long)h->group_tbm,
                                        (unsigned long long)b.nmatmax, (unsigned long long)b.ngkmax,
-                                       (unsigned long long)(uintptr_t)h->stream};
+                                       (unsigned long long)(uintptr_t)h->stream,
+                                       (unsigned long long)(uintptr_t)h->kinfo};
+  // a batch of other sizes (host buffers among them) may have moved a lane's workspace
+  for (int i = 0; i < L; ++i) k.push_back(h->lanes[i]->ws_gen);
   for (int i = 0; i < b.nk; ++i) {
     k.push_back((unsigned long long)b.nmatp[i]);
     k.push_back((unsigned long long)b.ngp[i]);
@@ -1627,7 +1631,7 @@ static void drop_graph(excfv_handle* h) {
 }
 
 // A device-pointer batch that repeats the previous call exactly (same sizes,
-// pointers, lanes, precision and per-SCF-iteration data) replays a CUDA graph
+// pointers, lanes and their workspaces, precision and per-SCF-iteration data) replays a CUDA graph
 // captured on its second occurrence; the first occurrence runs eagerly and
 // sizes every workspace.  If capture or instantiation fails, the batch runs
 // eagerly and capture is not tried again for this key.

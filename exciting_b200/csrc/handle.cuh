@@ -197,6 +197,7 @@ struct excfv_handle {
   int kinfo_cap = 0;
   int last_nk = 0;
   std::vector<int> batch_nmat;  // nmatp of the last batch (info offsets)
+  unsigned ws_gen = 0;          // incremented whenever the workspace is allocated anew
   unsigned static_gen = 0;      // incremented by every excfv_set_static
   // CUDA graph of the last device-pointer batch: its key (sizes, pointers,
   // lanes, precision, static generation), how often it ran eagerly, the

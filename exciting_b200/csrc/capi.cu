@@ -1611,7 +1611,9 @@ static std::vector<unsigned long long> batch_key(const excfv_handle* h, const Ba
                                        (unsigned long long)h->group_tbm,
                                        (unsigned long long)b.nmatmax, (unsigned long long)b.ngkmax,
                                        (unsigned long long)(uintptr_t)h->stream,
-                                       (unsigned long long)(uintptr_t)h->kinfo};
+                                       (unsigned long long)(uintptr_t)h->kinfo,
+                                       // excfv_hmlint can bring the IORA* terms, which take launches of their own
+                                       (unsigned long long)(h->st.have_h1aa ? (uintptr_t)h->st.h1aa : 0)};
   // a batch of other sizes (host buffers among them) may have moved a lane's workspace
   for (int i = 0; i < L; ++i) k.push_back(h->lanes[i]->ws_gen);
   for (int i = 0; i < b.nk; ++i) {

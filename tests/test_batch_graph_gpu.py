@@ -4,7 +4,9 @@ Repeated device-pointer batches replay a CUDA graph whose launches carry the
 addresses of the lanes' workspaces and of the status words.  Between two such
 batches a host-buffer batch with larger leading dimensions makes every lane
 allocate its workspace anew, and one with more k-points the status words; the
-device batch must then follow the new ones.  Bounds as in tests/test_batched_gpu.py.
+device batch must then follow the new ones.  The muffin-tin build can add the
+IORA* terms of the overlap, whose launches an earlier graph does not have.  Bounds
+as in tests/test_batched_gpu.py.
 """
 import numpy as np
 import pytest
@@ -81,3 +83,23 @@ def test_replay_after_the_workspaces_moved(mode):
             _check(refs * (len(kpts) // 3), p.kpts * (len(kpts) // 3), outs)
         for _ in range(3):
             _check(refs, p.kpts, b.run())
+
+
+def test_replay_after_the_muffin_tin_build():
+    p = syn.make_problem("diamond2", nk=3, ngk_range=(90, 140), nstfv=8, h1on=True)
+    st = p.static
+    st.h1aa[...], st.h1loa[...], st.h1lolo[...] = 0.0, 0.0, 0.0    # the build brings them
+    rad = syn.make_radial(st, nrmt=120, lmaxvr=4)
+    with FirstVariational(0) as fv:
+        fv.set_static(st)
+        fv.set_lanes(2)
+        b = _DeviceBatch(fv, p)
+        for _ in range(3):
+            before = b.run()
+        fv.hmlint(rad)
+        refs = [fv.seceqn(kp)[0] for kp in p.kpts]
+        for _ in range(3):
+            after = b.run()
+            for w_ref, (w, _) in zip(refs, after):
+                assert np.abs(w - w_ref).max() < 1e-10
+    assert max(np.abs(x[0] - y[0]).max() for x, y in zip(before, after)) > 1e-6   # the data did change

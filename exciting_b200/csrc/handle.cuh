@@ -266,6 +266,15 @@ int potrf_block();
 // diagonal block kb of every listed problem (each with n > kb), one CTA each
 int potrf_diag_grouped(cudaStream_t s, const PotrfProb* d_probs, int nprob, int kb);
 
+// A kernel's limit of dynamic shared memory is state of the process (per device),
+// and handles may run in different host threads: every kernel whose size depends on
+// the problem sets one constant, its largest, so that no thread lowers the limit
+// between another's call and its launch.
+template <typename K>
+cudaError_t raise_smem_limit(K* kernel, size_t largest) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)largest);
+}
+
 // ---- stages (each enqueues work on h->stream) ------------------------------
 int stage_reserve(excfv_handle* h, int nmatmax, int ngkmax, int kmax);
 // `bytes` of the handle's scratch.  Only for calls that synchronise the stream

@@ -138,6 +138,7 @@ constexpr int RK = 4;    // radial points per lane
 constexpr int JT = 4;    // states per warp step
 constexpr int PSI_T = 256;
 constexpr int PSI_R = 32 * RK;
+constexpr size_t PSI_SMEM = 200 * 1024;  // most dynamic shared memory
 
 __global__ void __launch_bounds__(PSI_T) k_rho_psi(RhoArgs a, int jc, const cplx* __restrict__ gang,
                                                    double* __restrict__ rtp) {
@@ -252,11 +253,11 @@ int rho_mt(excfv_handle* h, RhoArgs a) {
   const int fit = (int)(96 * 1024 / per);
   if (jc > fit) jc = std::max(JT, fit / 32 * 32);
   const size_t smem = per * jc;
-  if (smem > 200 * 1024) {
+  if (smem > PSI_SMEM) {
     excfv_set_error("rhovalk: %d radial functions per atom exceed the shared memory", nb);
     return EXCFV_ERR_UNSUPPORTED;
   }
-  CUDA_TRY(cudaFuncSetAttribute(k_rho_psi, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  CUDA_TRY(raise_smem_limit(k_rho_psi, PSI_SMEM));
   const size_t one = (size_t)a.nst * nb * L;
   const int group = (int)std::min<size_t>(a.natmtot, std::max<size_t>(1, h->rho.gang_elems / one));
   const int nj = (a.nst + ANG_T - 1) / ANG_T;
@@ -679,8 +680,7 @@ int stage_rhovalk_sv_nc(excfv_handle* h, int ngp, int ngkmax, const cplx* apwalm
   if ((rc = sv_spin(h, 0, evecsv, epsocc, d.coef2, d.lo2)) || (rc = sv_spin(h, 1, evecsv, epsocc, d.coef3, d.lo3)))
     return rc;
   const size_t smem = rho_nc_smem(d.lmmaxvr);
-  if (smem > 48 * 1024)
-    CUDA_TRY(cudaFuncSetAttribute(k_rho_mt_nc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  CUDA_TRY(raise_smem_limit(k_rho_mt_nc, rho_nc_smem((RHO_LMAX + 1) * (RHO_LMAX + 1))));
   dim3 grid(d.nrcmax, h->st.natmtot);
   k_rho_mt_nc<<<grid, 128, smem, s>>>(a, d.coef3, d.lo3, d.magmt3);
   count_launch();

@@ -27,6 +27,7 @@ namespace {
 // coefficients uncoalesced once per function.
 constexpr int LOJ = 8;    // functions per pass
 constexpr int LOW = 8;    // warps (G+k vectors) per CTA
+constexpr size_t LO_SMEM = 160 * 1024;  // most dynamic shared memory
 __global__ void __launch_bounds__(32 * LOW) k_lo_gk(int N, int natmtot, int maxaa, int maxnlo, int nlomax,
                                                     int apwordmax, const int* idxis, const int* lo_first,
                                                     const int* lo_lm, const int* lo_ilo, const int* fofl, int lmmax,
@@ -324,9 +325,9 @@ int stage_setup(excfv_handle* h, int nmatp, int ngp, bool mirror_o) {
   prof_begin(h, PROF_SETUP_OTHER);
   // local-orbital band (columns N..n-1)
   if (n > N) {
-    const bool staged = sizeof(cplx) * LOJ * st.maxaa <= 160 * 1024;
+    const bool staged = sizeof(cplx) * LOJ * st.maxaa <= LO_SMEM;
     const int smem = staged ? (int)(sizeof(cplx) * LOJ * st.maxaa) : 0;
-    CUDA_TRY(cudaFuncSetAttribute(k_lo_gk, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    CUDA_TRY(raise_smem_limit(k_lo_gk, LO_SMEM));
     const int gx = min((N + LOW - 1) / LOW, max(1, 8 * h->nsm / st.natmtot));
     k_lo_gk<<<dim3(gx, st.natmtot), 32 * LOW, smem, s>>>(N, st.natmtot, st.maxaa, st.maxnlo, st.nlomax, st.apwordmax,
                                                          st.idxis, st.lo_first, st.lo_lm, st.lo_ilo, st.fofl,

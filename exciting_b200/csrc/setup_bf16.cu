@@ -480,11 +480,7 @@ int zgemm_cn_bf16x(excfv_handle* h, int n, int K, const cplx* A, const cplx* Z, 
   a.flag = ws.status + ST_SETUP;
   a.wait_ns = wait_limit_ns();
   const size_t smem = (size_t)STAGES * STAGE_BYTES + 1024;
-  static bool attr = false;
-  if (!attr) {
-    CUDA_TRY(cudaFuncSetAttribute(k_zgemm_bf16x, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attr = true;
-  }
+  CUDA_TRY(raise_smem_limit(k_zgemm_bf16x, smem));
   k_zgemm_bf16x<<<2 * tpb, 32 * NWARP, smem, s>>>(a, mA, mA, mZ, mAb);
   count_launch();
   CUDA_TRY(cudaGetLastError());

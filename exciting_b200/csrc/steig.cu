@@ -263,6 +263,7 @@ __global__ void k_stein(int n, const double* __restrict__ d, const double* __res
 // is stored (a load does not pass a store that may alias it) and swaps are
 // selections.  k = 200, n = 1964: 639 -> 394 us; k = 20, n = 316: 108 -> 69 us.
 constexpr int SCH = 8;
+constexpr size_t STEIN_SMEM = 200 * 1024;  // most dynamic shared memory (order 5120)
 __global__ void __launch_bounds__(32) k_stein_smem(int n, const double* __restrict__ d,
                                                    const double* __restrict__ e,
                                                    const double* __restrict__ scal, int k,
@@ -457,8 +458,8 @@ int tridiag_eig(excfv_handle* h, int n, int k, double abstol, const double* d, c
   k_clusters<<<(k + 127) / 128, 128, 0, s>>>(k, w, scal, iscratch); count_launch();
   CUDA_TRY(cudaGetLastError());
   const size_t sbytes = 40 * (size_t)n;
-  if (sbytes <= 200 * 1024) {
-    CUDA_TRY(cudaFuncSetAttribute(k_stein_smem, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sbytes));
+  if (sbytes <= STEIN_SMEM) {
+    CUDA_TRY(raise_smem_limit(k_stein_smem, STEIN_SMEM));
     k_stein_smem<<<k, 32, sbytes, s>>>(n, d, e, scal, k, w, iscratch, Yi, h->ws.status); count_launch();
   } else {
     k_stein<<<(k + 31) / 32, 32, 0, s>>>(n, d, e, scal, k, w, iscratch, ua, ub, uf, um, Yi,

@@ -893,7 +893,7 @@ bool flow_shape(int n, int p, int G, FlowArgs<T2>& a, size_t* smem) {
 
 template <typename T2, int MC>
 int flow_panel(excfv_handle* h, const CUtensorMap& tmap, FlowArgs<T2> a, int G, size_t smem) {
-  CUDA_TRY(cudaFuncSetAttribute(k_tridiag_flow<T2, MC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  CUDA_TRY(raise_smem_limit(k_tridiag_flow<T2, MC>, FLOW_SMEM + 128));
   void* args[] = {&a, const_cast<CUtensorMap*>(&tmap)};
   CUDA_TRY(cudaLaunchCooperativeKernel((const void*)k_tridiag_flow<T2, MC>, dim3(G), dim3(FTOT), args, smem,
                                        h->stream));

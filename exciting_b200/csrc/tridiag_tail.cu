@@ -326,8 +326,7 @@ template <typename T2, int CL>
 cudaError_t tail_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* at, size_t smem, cudaStream_t s) {
   cudaError_t err = cudaSuccess;
   if (CL > 8) err = cudaFuncSetAttribute(k_tridiag_tail<T2, CL>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-  if (err == cudaSuccess)
-    err = cudaFuncSetAttribute(k_tridiag_tail<T2, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (err == cudaSuccess) err = raise_smem_limit(k_tridiag_tail<T2, CL>, SMEM_MAX);
   *cfg = cudaLaunchConfig_t{};
   cfg->gridDim = dim3(CL);
   cfg->blockDim = dim3(TT);

@@ -331,6 +331,41 @@ int stage_set_static(excfv_handle* h, const excfv_static* s) {
   return EXCFV_OK;
 }
 
+// The workspace's arrays for these sizes: returns the bytes of them all, and with
+// `place` sets their addresses inside ws.block.
+static size_t lay_out_workspace(const excfv_handle* h, Workspace& ws, int nmatmax, int ngkmax, int kmax, bool slices,
+                                bool place) {
+  const DevStatic& st = h->st;
+  const size_t n = nmatmax, n2 = n * n, AM = (size_t)st.natmtot * st.maxaa;
+  const size_t K = kmax;
+  // split-K scratch: up to 16 partial products of an n x n result, 8 M elements
+  // at most, and the back-transform's needs
+  ws.part_cap = std::max(std::min((size_t)(8u << 20), 16 * n2), n * 64 * 4);
+  // the slices of the precision form: A and aa A as BF16 slice planes (setup_bf16.cu)
+  ws.slices_elems = slices ? bf16x_plane_elems((int)AM, ngkmax) : 0;
+  ws.slice_sc_n = slices ? 2 * (size_t)bf16x_rpad(ngkmax) : 0;
+  size_t at = 0;
+  auto take = [&](auto** p, size_t count) {
+    if (place) *p = count ? reinterpret_cast<std::remove_reference_t<decltype(*p)>>(ws.block + at) : nullptr;
+    at += (count * sizeof(**p) + 255) / 256 * 256;
+  };
+  take(&ws.H, n2); take(&ws.O, n2); take(&ws.Ui, n2); take(&ws.T, n2);
+  take(&ws.Apk, AM * ngkmax); take(&ws.Zpk, AM * ngkmax);
+  take(&ws.ylm, (size_t)st.lmmaxapw * ngkmax);
+  take(&ws.djl, (size_t)ngkmax * (st.lmaxapw + 1) * st.apwordmax * st.nspecies);
+  take(&ws.apwalm, (size_t)ngkmax * st.apwordmax * st.lmmaxapw * st.natmtot);
+  take(&ws.igpig, (size_t)ngkmax); take(&ws.vgpc, (size_t)3 * ngkmax); take(&ws.gpc, (size_t)ngkmax);
+  take(&ws.tpgpc, (size_t)2 * ngkmax); take(&ws.sfacgp, (size_t)ngkmax * st.natmtot);
+  take(&ws.gk_iv, (size_t)3 * ngkmax); take(&ws.d, n); take(&ws.e, n); take(&ws.tau, n);
+  take(&ws.Wp, n * 4 * tridiag_nb()); take(&ws.red, (size_t)tridiag_workspace_doubles()); take(&ws.w, n);
+  take(&ws.stein_ws, tridiag_eig_scratch_doubles((int)n, (int)K)); take(&ws.icl, K); take(&ws.ybuf, 2 * n);
+  take(&ws.Z, n * K); take(&ws.Z2, n * K); take(&ws.Gk, K * K); take(&ws.Gki, K * K);
+  take(&ws.Tf, backtr_factor_elems((int)n)); take(&ws.Xs, 2 * 256 * K); take(&ws.status, (size_t)ST_NWORDS);
+  take(&ws.bar, (size_t)4); take(&ws.prog, n); take(&ws.flow, tridiag_flow_bytes((int)n, h->nsm));
+  take(&ws.part, ws.part_cap); take(&ws.slices, ws.slices_elems); take(&ws.slice_sc, ws.slice_sc_n);
+  return at;
+}
+
 int stage_reserve(excfv_handle* h, int nmatmax, int ngkmax, int kmax) {
   Workspace& ws = h->ws;
   if (!h->have_static) {
@@ -348,48 +383,15 @@ int stage_reserve(excfv_handle* h, int nmatmax, int ngkmax, int kmax) {
   cudaStreamSynchronize(h->stream);
   free_workspace(ws);
   h->ws_gen++;
-  const DevStatic& st = h->st;
-  const size_t n = nmatmax, n2 = n * n, AM = (size_t)st.natmtot * st.maxaa;
-  const size_t K = kmax;
-  // split-K scratch: up to 16 partial products of an n x n result, 8 M elements
-  // at most, and the back-transform's needs
-  ws.part_cap = std::max(std::min((size_t)(8u << 20), 16 * n2), n * 64 * 4);
-  // the slices of the precision form: A and aa A as BF16 slice planes (setup_bf16.cu)
-  ws.slices_elems = want_slices ? bf16x_plane_elems((int)AM, (int)ngkmax) : 0;
-  ws.slice_sc_n = want_slices ? 2 * (size_t)bf16x_rpad((int)ngkmax) : 0;
-  // All arrays in one allocation: two passes over the list, sizes and then
-  // addresses (order 715: 4.3 ms to reserve and 4.6 to free with an allocation per
-  // array, 0.38 and 1.2 like this).
-  size_t total = 0;
-  for (int pass = 0; pass < 2; ++pass) {
-    if (pass) {
-      const int rc = dalloc(&ws.block, total);
-      if (rc) {
-        free_workspace(ws);
-        return rc;
-      }
-    }
-    size_t at = 0;
-    auto take = [&](auto** p, size_t count) {
-      if (pass) *p = count ? reinterpret_cast<std::remove_reference_t<decltype(*p)>>(ws.block + at) : nullptr;
-      at += (count * sizeof(**p) + 255) / 256 * 256;
-    };
-    take(&ws.H, n2); take(&ws.O, n2); take(&ws.Ui, n2); take(&ws.T, n2);
-    take(&ws.Apk, AM * ngkmax); take(&ws.Zpk, AM * ngkmax);
-    take(&ws.ylm, (size_t)st.lmmaxapw * ngkmax);
-    take(&ws.djl, (size_t)ngkmax * (st.lmaxapw + 1) * st.apwordmax * st.nspecies);
-    take(&ws.apwalm, (size_t)ngkmax * st.apwordmax * st.lmmaxapw * st.natmtot);
-    take(&ws.igpig, (size_t)ngkmax); take(&ws.vgpc, (size_t)3 * ngkmax); take(&ws.gpc, (size_t)ngkmax);
-    take(&ws.tpgpc, (size_t)2 * ngkmax); take(&ws.sfacgp, (size_t)ngkmax * st.natmtot);
-    take(&ws.gk_iv, (size_t)3 * ngkmax); take(&ws.d, n); take(&ws.e, n); take(&ws.tau, n);
-    take(&ws.Wp, n * 4 * tridiag_nb()); take(&ws.red, (size_t)tridiag_workspace_doubles()); take(&ws.w, n);
-    take(&ws.stein_ws, tridiag_eig_scratch_doubles((int)n, (int)K)); take(&ws.icl, K); take(&ws.ybuf, 2 * n);
-    take(&ws.Z, n * K); take(&ws.Z2, n * K); take(&ws.Gk, K * K); take(&ws.Gki, K * K);
-    take(&ws.Tf, backtr_factor_elems((int)n)); take(&ws.Xs, 2 * 256 * K); take(&ws.status, (size_t)ST_NWORDS);
-    take(&ws.bar, (size_t)4); take(&ws.prog, n); take(&ws.flow, tridiag_flow_bytes((int)n, h->nsm));
-    take(&ws.part, ws.part_cap); take(&ws.slices, ws.slices_elems); take(&ws.slice_sc, ws.slice_sc_n);
-    total = at;
+  // All arrays in one allocation (order 715: 4.3 ms to reserve and 4.6 to free with
+  // an allocation per array, 0.38 and 1.2 like this).
+  const size_t total = lay_out_workspace(h, ws, nmatmax, ngkmax, kmax, want_slices, false);
+  if (const int rc = dalloc(&ws.block, total)) {
+    free_workspace(ws);
+    return rc;
   }
+  ws.bytes = total;
+  lay_out_workspace(h, ws, nmatmax, ngkmax, kmax, want_slices, true);
   // zeroed in the handle's stream order (lane streams do not wait for the legacy stream)
   CUDA_TRY(cudaMemsetAsync(ws.status, 0, ST_NWORDS * sizeof(int), h->stream));
   CUDA_TRY(cudaMemsetAsync(ws.bar, 0, 4 * sizeof(unsigned), h->stream));
@@ -1290,12 +1292,43 @@ static int enqueue_batch(excfv_handle* h, const BatchArgs& b, int L);
 static int run_batch_graph(excfv_handle* h, const BatchArgs& b, int L);
 static void group_segments(excfv_handle* h, const BatchArgs& b, int L, std::vector<std::vector<int>>& segs);
 
-// Enqueues the whole batch on L lanes (largest k-points first, each to the
-// least-loaded lane), fork/join on h->stream.
+// Lanes of a batch when the caller has chosen none.  Orders that the cluster
+// kernel reduces alone in clusters of 8 have no cooperative panels to share the
+// SMs out to: up to 32 lanes, all k-points of most batches at once (28 k-points of
+// order ~300: 8 lanes 10.5 ms, 16 8.9, 28 6.1).  A lane's workspace is sized by the
+// caller's nmatmax, whatever the batch's orders: more than 8 lanes only while all of
+// them take at most a quarter of the memory that is free or already theirs.
+static int default_lanes(excfv_handle* h, const BatchArgs& b, int nmax) {
+  if (h->nlanes_pref > 0) return h->nlanes_pref;
+  const bool tail_alone = nmax <= tridiag_tail_lane_max(h->prec == EXCFV_PREC_MIXED);
+  const int most = std::min({tail_alone ? 32 : 8, (int)b.nk, max_lanes_for(h, nmax)});
+  if (most <= 8) return most;
+  const bool mixed = h->prec == EXCFV_PREC_MIXED;
+  int kmax = std::max(1, h->st.nstfv);
+  if (mixed) kmax = mixed_states(b.nmatmax, kmax);
+  size_t held = 0;
+  int ready = 0;  // lanes that need no allocation
+  for (int i = 0; i < (int)h->lanes.size(); ++i) {
+    const Workspace& ws = h->lanes[i]->ws;
+    held += ws.bytes;
+    if (i < most && ws.H && b.nmatmax <= ws.nmatmax && b.ngkmax == ws.ngkmax && kmax <= ws.kmax && (!mixed || ws.slices))
+      ++ready;
+  }
+  if (ready == most) return most;
+  Workspace sizes;
+  const size_t per = lay_out_workspace(h, sizes, b.nmatmax, b.ngkmax, kmax, mixed, false);
+  size_t fr = 0, tot = 0;
+  if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) return 8;
+  return (int)std::max<size_t>(8, std::min<size_t>(most, (fr + held) / 4 / per));
+}
+
+// Enqueues the whole batch on L lanes (0: default_lanes; largest k-points first,
+// each to the least-loaded lane), fork/join on h->stream.
 static int run_batch(excfv_handle* h, const BatchArgs& b, int L) {
   int nmax = 0;
   int rc = check_batch(h, b, &nmax);
   if (rc) return rc;
+  if (L <= 0) L = default_lanes(h, b, nmax);
   L = std::max(1, std::min(L, std::min(b.nk, max_lanes_for(h, nmax))));
   if ((rc = ensure_lanes(h, L, b.nmatmax, b.ngkmax, std::max(1, h->st.nstfv)))) return rc;
   if (h->kinfo_cap < b.nk) {
@@ -1683,18 +1716,6 @@ static BatchArgs make_batch(int32_t nk, const int32_t* nmatp, const int32_t* ngp
   return b;
 }
 
-// Lanes of a batch when the caller has chosen none.  Orders that the cluster
-// kernel reduces alone in clusters of 8 have no cooperative panels to share the
-// SMs out to: up to 32 lanes, all k-points of most batches at once (28 k-points of
-// order ~300: 8 lanes 10.5 ms, 16 8.9, 28 6.1).
-static int default_lanes(excfv_handle* h, const BatchArgs& b) {
-  if (h->nlanes_pref > 0) return h->nlanes_pref;
-  int nmax = 0;
-  for (int k = 0; k < b.nk; ++k) nmax = std::max(nmax, (int)b.nmatp[k]);
-  const int most = nmax <= tridiag_tail_lane_max(h->prec == EXCFV_PREC_MIXED) ? 32 : 8;
-  return std::min(most, max_lanes_for(h, nmax));
-}
-
 int excfv_seceqn_batched_dev(excfv_handle* h, int32_t nk, const int32_t* nmatp, const int32_t* ngp,
                              int32_t ngkmax, const double* const* gpc, const double* const* tpgpc,
                              const double* const* sfacgp, const int32_t* const* igpig,
@@ -1704,7 +1725,7 @@ int excfv_seceqn_batched_dev(excfv_handle* h, int32_t nk, const int32_t* nmatp, 
   DeviceGuard g(h->device);
   BatchArgs b = make_batch(nk, nmatp, ngp, ngkmax, gpc, tpgpc, sfacgp, igpig, vgpc, nmatmax, evalfv,
                            evecfv, false);
-  return run_batch(h, b, default_lanes(h, b));
+  return run_batch(h, b, 0);
 }
 
 int excfv_seceqn_batched(excfv_handle* h, int32_t nk, const int32_t* nmatp, const int32_t* ngp,
@@ -1716,7 +1737,7 @@ int excfv_seceqn_batched(excfv_handle* h, int32_t nk, const int32_t* nmatp, cons
   DeviceGuard g(h->device);
   BatchArgs b = make_batch(nk, nmatp, ngp, ngkmax, gpc, tpgpc, sfacgp, igpig, vgpc, nmatmax, evalfv,
                            evecfv, true);
-  int rc = run_batch(h, b, default_lanes(h, b));
+  int rc = run_batch(h, b, 0);
   if (rc) return rc;
   return batch_info(h, nk, info);
 }

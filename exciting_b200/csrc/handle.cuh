@@ -57,6 +57,7 @@ struct DevStatic {
 
 struct Workspace {
   unsigned char* block = nullptr;  // the allocation that holds every array below
+  size_t bytes = 0;                // its size
   int nmatmax = 0, ngkmax = 0, kmax = 0;
   cplx* H = nullptr;        // n x n
   cplx* O = nullptr;        // n x n

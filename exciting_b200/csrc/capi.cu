@@ -29,6 +29,7 @@ int dalloc(T** p, size_t count) {
   cudaError_t e = cudaMalloc((void**)p, count * sizeof(T));
   if (e != cudaSuccess) {
     excfv_set_error("cudaMalloc of %zu bytes failed: %s", count * sizeof(T), cudaGetErrorString(e));
+    (void)cudaGetLastError();
     *p = nullptr;
     return EXCFV_ERR_ALLOC;
   }
@@ -137,6 +138,7 @@ int handle_scratch(excfv_handle* h, size_t bytes, void** p) {
     cudaError_t e = cudaMalloc(&h->scratch, bytes);
     if (e != cudaSuccess) {
       excfv_set_error("cudaMalloc of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
+      (void)cudaGetLastError();
       h->scratch = nullptr;
       return EXCFV_ERR_ALLOC;
     }

@@ -45,12 +45,15 @@ EXCFV_HD double cabs2(cplx a) { return a.x * a.x + a.y * a.y; }
 //       setup, not by the eigensolve)
 enum { ST_POTRF = 0, ST_BARRIER = 1, ST_STEIN = 2, ST_STEBZ = 3, ST_REFINE = 4, ST_SETUP = 5, ST_NWORDS = 8 };
 
+// The error is taken off the runtime's record: left there, a failed allocation
+// would come back from the check after the next call's first launch.
 #define CUDA_TRY(expr)                                                          \
   do {                                                                          \
     cudaError_t _e = (expr);                                                    \
     if (_e != cudaSuccess) {                                                    \
       excfv_set_error("%s:%d: %s: %s", __FILE__, __LINE__, #expr,               \
                       cudaGetErrorString(_e));                                  \
+      (void)cudaGetLastError();                                                 \
       return EXCFV_ERR_CUDA;                                                    \
     }                                                                           \
   } while (0)

@@ -273,6 +273,7 @@ int stage_set_bfield(excfv_handle* h, const excfv_bfield* b) {
   const size_t nlo1 = std::max(st.maxnlo, 1), nst = std::max(st.nstfv, 1);
   auto al = [](auto** p, size_t n) -> int {
     if (cudaMalloc(p, sizeof(**p) * std::max<size_t>(n, 1)) != cudaSuccess) {
+      (void)cudaGetLastError();
       excfv_set_error("excfv_set_bfield: cudaMalloc failed");
       return EXCFV_ERR_ALLOC;
     }
@@ -306,6 +307,7 @@ namespace {
 template <typename T>
 int sv_alloc(T** p, size_t n) {
   if (cudaMalloc(p, sizeof(T) * std::max<size_t>(n, 1)) != cudaSuccess) {
+    (void)cudaGetLastError();
     excfv_set_error("excfv_set_bfield_nc: cudaMalloc failed");
     return EXCFV_ERR_ALLOC;
   }

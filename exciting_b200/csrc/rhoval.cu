@@ -259,7 +259,9 @@ int rho_mt(excfv_handle* h, RhoArgs a) {
   }
   CUDA_TRY(raise_smem_limit(k_rho_psi, PSI_SMEM));
   const size_t one = (size_t)a.nst * nb * L;
-  const int group = (int)std::min<size_t>(a.natmtot, std::max<size_t>(1, h->rho.gang_elems / one));
+  // (k_rho_ang's grid has a row per function and atom, 65535 at most)
+  const int group = (int)std::min<size_t>(std::min(a.natmtot, std::max(1, 65535 / nb)),
+                                          std::max<size_t>(1, h->rho.gang_elems / one));
   const int nj = (a.nst + ANG_T - 1) / ANG_T;
   for (a.ias0 = 0; a.ias0 < a.natmtot; a.ias0 += group) {
     const int na = std::min(group, a.natmtot - a.ias0);

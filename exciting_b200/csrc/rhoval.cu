@@ -133,13 +133,15 @@ __global__ void __launch_bounds__(ANG_T) k_rho_ang(RhoArgs a, cplx* __restrict__
 // of states is copied to shared memory; a lane owns radial points r, r+32, ...;
 // a warp takes JT states at a time (g broadcast, u coalesced from L1), so each u
 // or g loaded feeds JT or RK complex FMAs, and |psi|^2 stays in registers.
-// Bound by FP64 FMAs.
+// Bound by FP64 FMAs.  STAGED false: more functions than shared memory holds for a
+// warp's states; g is read where it is.
 constexpr int RK = 4;    // radial points per lane
 constexpr int JT = 4;    // states per warp step
 constexpr int PSI_T = 256;
 constexpr int PSI_R = 32 * RK;
 constexpr size_t PSI_SMEM = 200 * 1024;  // most dynamic shared memory
 
+template <bool STAGED>
 __global__ void __launch_bounds__(PSI_T) k_rho_psi(RhoArgs a, int jc, const cplx* __restrict__ gang,
                                                    double* __restrict__ rtp) {
   extern __shared__ __align__(16) unsigned char dsm[];
@@ -156,20 +158,25 @@ __global__ void __launch_bounds__(PSI_T) k_rho_psi(RhoArgs a, int jc, const cplx
   const cplx* gin = gang + (size_t)a.nst * nb * (tp + (size_t)L * blockIdx.y);
   for (int j0 = 0; j0 < a.nst; j0 += jc) {
     const int nj = min(jc, a.nst - j0);
-    __syncthreads();
-    for (int b = warp; b < nb; b += PSI_T / 32)
-      for (int jj = lane; jj < jc; jj += 32) g[b * jc + jj] = (jj < nj) ? gin[j0 + jj + (size_t)a.nst * b] : cmk(0.0, 0.0);
-    __syncthreads();
+    if constexpr (STAGED) {
+      __syncthreads();
+      for (int b = warp; b < nb; b += PSI_T / 32)
+        for (int jj = lane; jj < jc; jj += 32) g[b * jc + jj] = (jj < nj) ? gin[j0 + jj + (size_t)a.nst * b] : cmk(0.0, 0.0);
+      __syncthreads();
+    }
     for (int jj = JT * warp; jj < nj; jj += JT * (PSI_T / 32)) {  // jc is a multiple of JT
       cplx psi[RK][JT];
 #pragma unroll
       for (int k = 0; k < RK; ++k)
 #pragma unroll
         for (int t = 0; t < JT; ++t) psi[k][t] = cmk(0.0, 0.0);
-      auto add = [&](const double* ub, const cplx* gb) {
+      auto add = [&](const double* ub, int b) {
         cplx gv[JT];
 #pragma unroll
-        for (int t = 0; t < JT; ++t) gv[t] = gb[t];
+        for (int t = 0; t < JT; ++t) {
+          if constexpr (STAGED) gv[t] = g[b * jc + jj + t];
+          else gv[t] = (jj + t < nj) ? gin[j0 + jj + t + (size_t)a.nst * b] : cmk(0.0, 0.0);
+        }
 #pragma unroll
         for (int k = 0; k < RK; ++k) {
           const int r = r0 + lane + 32 * k;
@@ -183,9 +190,9 @@ __global__ void __launch_bounds__(PSI_T) k_rho_psi(RhoArgs a, int jc, const cplx
       };
       const double* ua = a.ucoarse + (size_t)a.nrcmax * na * ias;
 #pragma unroll 2
-      for (int b = 0; b < na; ++b) add(ua + (size_t)a.nrcmax * b, g + b * jc + jj);
+      for (int b = 0; b < na; ++b) add(ua + (size_t)a.nrcmax * b, b);
       const double* va = a.vcoarse + (size_t)a.nrcmax * a.nlomax * ias;
-      for (int b = na; b < nb; ++b) add(va + (size_t)a.nrcmax * (b - na), g + b * jc + jj);
+      for (int b = na; b < nb; ++b) add(va + (size_t)a.nrcmax * (b - na), b);
 #pragma unroll
       for (int t = 0; t < JT; ++t) {
         const double wj = (jj + t < nj) ? a.w[j0 + jj + t] : 0.0;
@@ -252,12 +259,10 @@ int rho_mt(excfv_handle* h, RhoArgs a) {
   const size_t per = sizeof(cplx) * nb;
   const int fit = (int)(96 * 1024 / per);
   if (jc > fit) jc = std::max(JT, fit / 32 * 32);
-  const size_t smem = per * jc;
-  if (smem > PSI_SMEM) {
-    excfv_set_error("rhovalk: %d radial functions per atom exceed the shared memory", nb);
-    return EXCFV_ERR_UNSUPPORTED;
-  }
-  CUDA_TRY(raise_smem_limit(k_rho_psi, PSI_SMEM));
+  const bool staged = per * jc <= PSI_SMEM;
+  const size_t smem = staged ? per * jc : 0;
+  CUDA_TRY(raise_smem_limit(k_rho_psi<true>, PSI_SMEM));
+  auto* psi = staged ? k_rho_psi<true> : k_rho_psi<false>;
   const size_t one = (size_t)a.nst * nb * L;
   // (k_rho_ang's grid has a row per function and atom, 65535 at most)
   const int group = (int)std::min<size_t>(std::min(a.natmtot, std::max(1, 65535 / nb)),
@@ -269,7 +274,7 @@ int rho_mt(excfv_handle* h, RhoArgs a) {
     const int tz = std::min(L, std::max(1, 4 * h->nsm / (nj * nb * na)));
     k_rho_ang<<<dim3(nj, nb * na, tz), ANG_T, 0, s>>>(a, gang);
     count_launch();
-    k_rho_psi<<<dim3(L, na, (a.nrcmax + PSI_R - 1) / PSI_R), PSI_T, smem, s>>>(a, jc, gang, rtp);
+    psi<<<dim3(L, na, (a.nrcmax + PSI_R - 1) / PSI_R), PSI_T, smem, s>>>(a, jc, gang, rtp);
     count_launch();
   }
   k_rho_sht<<<dim3((a.nrcmax + SHT_R - 1) / SHT_R, a.natmtot), 256, 0, s>>>(a, rtp);

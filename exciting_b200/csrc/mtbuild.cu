@@ -159,12 +159,12 @@ void gauss_legendre(int n, std::vector<double>& xq, std::vector<double>& wq) {
   }
 }
 
-// Quadrature nodes of the Gaunt coefficients: weights times 2 pi, then
-// Y_lm (real at phi = 0) of every node, lm up to max(lmaxmat, lmaxvr).
-int gaunt_nodes(int lmaxmat, int lmaxvr) { return (2 * lmaxmat + lmaxvr) / 2 + 2; }
-void gaunt_node_values(int lmaxmat, int lmaxvr, double* out) {
-  const int L = std::max(lmaxmat, lmaxvr), lmL = (L + 1) * (L + 1);
-  const int nq = gaunt_nodes(lmaxmat, lmaxvr);
+// Quadrature nodes of the Gaunt coefficients for l1, l3 <= lg: weights times 2 pi,
+// then Y_lm (real at phi = 0) of every node, lm up to max(lg, lmaxvr).
+int gaunt_nodes(int lg, int lmaxvr) { return (2 * lg + lmaxvr) / 2 + 2; }
+void gaunt_node_values(int lg, int lmaxvr, double* out) {
+  const int L = std::max(lg, lmaxvr), lmL = (L + 1) * (L + 1);
+  const int nq = gaunt_nodes(lg, lmaxvr);
   std::vector<double> xq, wq;
   gauss_legendre(nq, xq, wq);
   std::vector<cplx> y(lmL);
@@ -190,7 +190,8 @@ struct MtArgs {
   const double* veff;   // (lmvr, nrmtmax, natmtot)
   double a;             // ZORA: alpha^2 / 2 (0 without valence relativity)
   int lmaxvr, nspecies;
-  const double* gnt;    // (lmaxvr+1, lmmat, lmmat): integral conj(Y_lm1) Y_(l2, m1-m3) Y_lm3
+  int lg;               // largest l of the APWs and local orbitals
+  const double* gnt;    // (lmaxvr+1, (lg+1)^2, (lg+1)^2): integral conj(Y_lm1) Y_(l2, m1-m3) Y_lm3
 };
 
 __device__ __forceinline__ int l_of(int lm) {
@@ -202,14 +203,14 @@ __device__ __forceinline__ int l_of(int lm) {
 
 // gnt(l2, lm3, lm1) from the quadrature nodes y (gaunt_node_values), one
 // thread per entry; exact zeros by the triangle rule and parity
-__global__ void k_gaunt(int lmaxmat, int lmaxvr, int nq, const double* __restrict__ y, double* __restrict__ gnt) {
-  const int lmmat = (lmaxmat + 1) * (lmaxmat + 1);
-  const int L = max(lmaxmat, lmaxvr), lmL = (L + 1) * (L + 1);
+__global__ void k_gaunt(int lg, int lmaxvr, int nq, const double* __restrict__ y, double* __restrict__ gnt) {
+  const int lmg = (lg + 1) * (lg + 1);
+  const int L = max(lg, lmaxvr), lmL = (L + 1) * (L + 1);
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (long long)lmmat * lmmat * (lmaxvr + 1)) return;
+  if (t >= (long long)lmg * lmg * (lmaxvr + 1)) return;
   const int l2 = (int)(t % (lmaxvr + 1));
-  const int lm3 = (int)((t / (lmaxvr + 1)) % lmmat);
-  const int lm1 = (int)(t / ((long long)(lmaxvr + 1) * lmmat));
+  const int lm3 = (int)((t / (lmaxvr + 1)) % lmg);
+  const int lm1 = (int)(t / ((long long)(lmaxvr + 1) * lmg));
   const int l1 = l_of(lm1), l3 = l_of(lm3);
   const int m2 = (lm1 - l1 * (l1 + 1)) - (lm3 - l3 * (l3 + 1));
   double s = 0.0;
@@ -228,9 +229,9 @@ __global__ void k_gaunt(int lmaxmat, int lmaxvr, int nq, const double* __restric
 // m2 = M, -M contribute: R_lm2 = (Y_lm2 + (-1)^m Y_l2,-m2)/sqrt 2 for m2 > 0,
 // -i (Y_lm2 - (-1)^m Y_l2,-m2)/sqrt 2 for m2 < 0, Y_l2,0 for m2 = 0.
 __device__ __forceinline__ cplx gaunt_sum(const MtArgs& m, int lm1, int l1, int lm3, int l3, const double* h) {
-  const int lmmat = (m.lmaxmat + 1) * (m.lmaxmat + 1);
+  const int lmg = (m.lg + 1) * (m.lg + 1);
   const int M = (lm1 - l1 * (l1 + 1)) - (lm3 - l3 * (l3 + 1)), am = abs(M);
-  const double* g = m.gnt + ((size_t)lm1 * lmmat + lm3) * (m.lmaxvr + 1);
+  const double* g = m.gnt + ((size_t)lm1 * lmg + lm3) * (m.lmaxvr + 1);
   const double sg = (am & 1) ? -1.0 : 1.0, sh = sqrt(0.5);
   const double fx = (M > 0) ? sh : sh * sg;      // factor of h(l2, |M|)
   const double fy = (M > 0) ? sh * sg : -sh;     // factor of i h(l2, -|M|)
@@ -522,7 +523,10 @@ static int mt_build(excfv_handle* h, const excfv_mtrad* r, const double* pot, bo
   const int L1 = st.lmaxmat + 1;
   // host: spline weights (times r^2) per species, the Gaunt quadrature nodes
   // and the species' local-orbital lists, in one block for one upload
-  const int lmmat = L1 * L1, lmL = std::max(lmmat, lmvr), nq = gaunt_nodes(st.lmaxmat, r->lmaxvr);
+  int lg = st.lmaxmat;
+  for (int is = 0; is < st.nspecies; ++is)
+    for (int ilo = 0; ilo < nlorb_h[is]; ++ilo) lg = std::max(lg, lorbl_h[ilo + (size_t)nlomax * is]);
+  const int lmg = (lg + 1) * (lg + 1), lmL = std::max(lmg, lmvr), nq = gaunt_nodes(lg, r->lmaxvr);
   const size_t nr2 = (size_t)r->nrmtmax, N = st.natmtot;
   const size_t n_mesh = nr2 * st.nspecies, n_node = (size_t)nq * (lmL + 1);
   const size_t n_int = ((size_t)(2 + nlomax) * st.nspecies + 1) / 2;  // ints, in doubles
@@ -544,13 +548,13 @@ static int mt_build(excfv_handle* h, const excfv_mtrad* r, const double* pot, bo
       ints[(2 + ilo) * st.nspecies + is] = lorbl_h[ilo + (size_t)nlomax * is];
   }
   std::copy(r->spr, r->spr + n_mesh, pack.begin() + n_mesh);
-  gaunt_node_values(st.lmaxmat, r->lmaxvr, pack.data() + 2 * n_mesh);
+  gaunt_node_values(lg, r->lmaxvr, pack.data() + 2 * n_mesh);
   // device: inputs and integrals in the handle's scratch
   const int A = st.apwordmax;
   const int per_aa = L1 * A * L1 * A * lmvr, per_loa = nlomax * L1 * A * lmvr, per_lolo = nlomax * nlomax * lmvr;
   const int per_kaa = L1 * A * A, per_kalo = nlomax * A, per_klolo = nlomax * nlomax;
   const size_t n_apw = nr2 * 2 * A * (st.lmaxapw + 1) * N, n_lo = nr2 * 2 * nlomax * N, n_v = (size_t)lmvr * nr2 * N;
-  const size_t n_gnt = (size_t)lmmat * lmmat * (r->lmaxvr + 1);
+  const size_t n_gnt = (size_t)lmg * lmg * (r->lmaxvr + 1);
   size_t total = 0;
   auto take = [&](size_t n) { const size_t at = total; total += (n + 31) / 32 * 32; return at; };
   const size_t o_pack = take(pack.size()), o_apw = take(n_apw), o_lo = take(n_lo), o_v = take(n_v),
@@ -569,7 +573,7 @@ static int mt_build(excfv_handle* h, const excfv_mtrad* r, const double* pot, bo
   m.natmtot = st.natmtot; m.lmaxmat = st.lmaxmat; m.lmaxapw = st.lmaxapw; m.apwordmax = st.apwordmax;
   m.nlomax = nlomax; m.lmvr = lmvr; m.nrmtmax = r->nrmtmax; m.maxaa = st.maxaa; m.maxnlo = std::max(st.maxnlo, 1);
   m.a = (st.vrel != 0) ? 0.5 * ALPHA_FS * ALPHA_FS : 0.0;
-  m.lmaxvr = r->lmaxvr; m.nspecies = st.nspecies;
+  m.lmaxvr = r->lmaxvr; m.lg = lg; m.nspecies = st.nspecies;
   m.idxis = st.idxis; m.apword = st.apword;
   const int* d_ints = reinterpret_cast<const int*>(D + o_pack + 2 * n_mesh + n_node);
   m.nrmt = d_ints; m.nlorb = d_ints + st.nspecies; m.lorbl = d_ints + 2 * st.nspecies;
@@ -587,7 +591,7 @@ static int mt_build(excfv_handle* h, const excfv_mtrad* r, const double* pot, bo
   }
   {
     auto grid = [](long long n) { return (unsigned)((n + 127) / 128); };
-    k_gaunt<<<grid((long long)n_gnt), 128, 0, s>>>(st.lmaxmat, r->lmaxvr, nq, D + o_pack + 2 * n_mesh, D + o_gnt);
+    k_gaunt<<<grid((long long)n_gnt), 128, 0, s>>>(lg, r->lmaxvr, nq, D + o_pack + 2 * n_mesh, D + o_gnt);
     count_launch();
     RadSets sets;
     sets.n = 0;

@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(32 * LOW) k_lo_gk(int N, int natmtot, int maxa
         const int jj = q0 + q, lm = lo_lm[jj + maxnlo * a];
         if (lm < 0) continue;  // the atom has fewer functions
         cplx ov = cmk(0.0, 0.0);
-        for (int io = 0; io < apwordmax; ++io) {
+        for (int io = 0; lm < lmmax && io < apwordmax; ++io) {  // no APW has l above lmaxapw
           const int f = fofl[(lm * apwordmax + io) + lmmax * apwordmax * is];
           if (f < 0) continue;
           const cplx y = ac[f];

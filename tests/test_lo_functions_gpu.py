@@ -5,7 +5,7 @@ The local-orbital band takes an atom's functions eight at a time and a warp per
 G+k vector, and the matching coefficients a thread per G+k vector and order: an
 incomplete pass, two passes, and G+k counts that do not fill the last blocks.
 Each entry is one sum of maxaa products, so 1e-13 of the largest entry as for
-the path's other setups.
+the path's other setups.  An orbital above lmaxapw overlaps no APW.
 """
 import dataclasses
 
@@ -59,3 +59,18 @@ def test_setup(ls, ngk, shape):
     up = np.triu(np.ones(H.shape, dtype=bool))
     assert np.abs(h - H)[up].max() < 1e-13 * np.abs(H).max()
     assert np.abs(o - O)[up].max() < 1e-13 * np.abs(O).max()
+
+
+def test_orbital_above_lmaxapw():
+    p = syn.make_problem("diamond2", ngk=61, nstfv=4, lmaxapw=2)
+    st, kp = _with_orbitals(p.static, (1, 4)), p.kpts[0]
+    A = fvref.match(st, kp)
+    with FirstVariational(0) as fv:
+        fv.set_static(st)
+        h, o = fv.hamiltonandoverlapsetup(kp, fv.match(kp))
+    N, nfun = kp.ngp, st.maxnlo
+    for a in range(st.natmtot):
+        cols = slice(N + nfun * a, N + nfun * (a + 1))
+        want = np.conj(st.loa[:, :, a] @ fvref._apwi(st, A, a, N)).T
+        assert np.abs(h[:N, cols] - want).max() < 1e-13 * np.abs(h).max()
+        assert np.abs(o[:N, cols][:, :3]).max() > 0 and not o[:N, cols][:, 3:].any()

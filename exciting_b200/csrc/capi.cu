@@ -368,6 +368,13 @@ static size_t lay_out_workspace(const excfv_handle* h, Workspace& ws, int nmatma
   return at;
 }
 
+// Whether a workspace has room for these sizes in the handle's basis.
+static bool workspace_holds(const excfv_handle* h, const Workspace& ws, int nmatmax, int ngkmax, int kmax,
+                            bool slices) {
+  return ws.H && nmatmax <= ws.nmatmax && ngkmax <= ws.ngkmax && kmax <= ws.kmax && (!slices || ws.slices) &&
+         ws.basis.holds(Basis(h->st));
+}
+
 int stage_reserve(excfv_handle* h, int nmatmax, int ngkmax, int kmax) {
   Workspace& ws = h->ws;
   if (!h->have_static) {
@@ -377,8 +384,7 @@ int stage_reserve(excfv_handle* h, int nmatmax, int ngkmax, int kmax) {
   // the precision form carries extra states through the eigensolver
   if (h->prec == EXCFV_PREC_MIXED) kmax = mixed_states(nmatmax, kmax);
   const bool want_slices = (h->prec == EXCFV_PREC_MIXED);
-  if (nmatmax <= ws.nmatmax && ngkmax <= ws.ngkmax && kmax <= ws.kmax && ws.H && (!want_slices || ws.slices))
-    return EXCFV_OK;
+  if (workspace_holds(h, ws, nmatmax, ngkmax, kmax, want_slices)) return EXCFV_OK;
   nmatmax = std::max(nmatmax, ws.nmatmax);
   ngkmax = std::max(ngkmax, ws.ngkmax);
   kmax = std::max(kmax, ws.kmax);
@@ -400,6 +406,7 @@ int stage_reserve(excfv_handle* h, int nmatmax, int ngkmax, int kmax) {
   ws.nmatmax = (int)nmatmax;
   ws.ngkmax = (int)ngkmax;
   ws.kmax = (int)kmax;
+  ws.basis = Basis(h->st);
   return EXCFV_OK;
 }
 
@@ -1313,8 +1320,7 @@ static int default_lanes(excfv_handle* h, const BatchArgs& b, int nmax) {
   for (int i = 0; i < (int)h->lanes.size(); ++i) {
     const Workspace& ws = h->lanes[i]->ws;
     held += ws.bytes;
-    if (i < most && ws.H && b.nmatmax <= ws.nmatmax && b.ngkmax == ws.ngkmax && kmax <= ws.kmax && (!mixed || ws.slices))
-      ++ready;
+    if (i < most && b.ngkmax == ws.ngkmax && workspace_holds(h, ws, b.nmatmax, b.ngkmax, kmax, mixed)) ++ready;
   }
   if (ready == most) return most;
   Workspace sizes;

@@ -55,10 +55,25 @@ struct DevStatic {
   int* gkcount = nullptr;   // per-block counts of the G+k compaction, then ngp and overflow
 };
 
+// The sizes of the basis that arrays outside DevStatic are dimensioned by; another
+// excfv_set_static can change them.
+struct Basis {
+  int natmtot = 0, nspecies = 0, lmaxapw = 0, apwordmax = 0, maxaa = 0;
+  Basis() = default;
+  explicit Basis(const DevStatic& st)
+      : natmtot(st.natmtot), nspecies(st.nspecies), lmaxapw(st.lmaxapw), apwordmax(st.apwordmax), maxaa(st.maxaa) {}
+  // whether arrays of these sizes have room for those of b
+  bool holds(const Basis& b) const {
+    return b.natmtot <= natmtot && b.nspecies <= nspecies && b.lmaxapw <= lmaxapw && b.apwordmax <= apwordmax &&
+           b.maxaa <= maxaa;
+  }
+};
+
 struct Workspace {
   unsigned char* block = nullptr;  // the allocation that holds every array below
   size_t bytes = 0;                // its size
   int nmatmax = 0, ngkmax = 0, kmax = 0;
+  Basis basis;
   cplx* H = nullptr;        // n x n
   cplx* O = nullptr;        // n x n
   cplx* Ui = nullptr;       // n x n, inverse Cholesky factor

@@ -585,10 +585,17 @@ static int rho_stage_k(excfv_handle* h, int ngp, int ngkmax, int nmatmax, const 
   return stage_match(h, ngp, ngkmax, apwalm ? ws.apwalm : nullptr);
 }
 
+// atoms that the density's accumulators and the caller's arrays both have
+static size_t rho_atoms(const excfv_handle* h) { return std::min(h->rho.basis.natmtot, h->st.natmtot); }
+
 static int check_rho(excfv_handle* h, int ngp, int ngkmax, int nmatmax) {
   if (!h) return EXCFV_ERR_ARG;
   if (!h->have_static || !h->rho.ready) {
     excfv_set_error("excfv_set_static and excfv_set_rho must be called first");
+    return EXCFV_ERR_STATE;
+  }
+  if (!h->rho.basis.serves(Basis(h->st)) || h->rho.lmaxvr > h->st.lmaxapw) {
+    excfv_set_error("excfv_set_rho must be called again: excfv_set_static has changed the basis");
     return EXCFV_ERR_STATE;
   }
   if (ngp <= 0 || ngp > ngkmax || nmatmax < ngp + h->st.nlotot) {
@@ -674,6 +681,10 @@ static int check_sv(excfv_handle* h, int ngp, int ngkmax, int nmatmax) {
   if (!h) return EXCFV_ERR_ARG;
   if (!h->have_static || !h->sv.ready) {
     excfv_set_error("excfv_set_static and excfv_set_bfield must be called first");
+    return EXCFV_ERR_STATE;
+  }
+  if (!h->sv.basis.serves(Basis(h->st))) {
+    excfv_set_error("excfv_set_bfield must be called again: excfv_set_static has changed the basis");
     return EXCFV_ERR_STATE;
   }
   if (ngp <= 0 || ngp > ngkmax || nmatmax < ngp + h->st.nlotot || h->st.nstfv > ngp) {
@@ -767,7 +778,7 @@ int excfv_get_magmt3(excfv_handle* h, double* magmt, int32_t reset) {
     return EXCFV_ERR_STATE;
   }
   DeviceGuard g(h->device);
-  const size_t n = (size_t)3 * h->rho.lmmaxvr * h->rho.nrmtmax * h->st.natmtot;
+  const size_t n = (size_t)3 * h->rho.lmmaxvr * h->rho.nrmtmax * rho_atoms(h);
   if (magmt) CUDA_TRY(cudaMemcpyAsync(magmt, h->rho.magmt3, sizeof(double) * n, cudaMemcpyDeviceToHost, h->stream));
   if (reset) CUDA_TRY(cudaMemsetAsync(h->rho.magmt3, 0, sizeof(double) * n, h->stream));
   CUDA_TRY(cudaStreamSynchronize(h->stream));
@@ -781,7 +792,7 @@ int excfv_get_magmt(excfv_handle* h, double* magmt, int32_t reset) {
     return EXCFV_ERR_STATE;
   }
   DeviceGuard g(h->device);
-  const size_t n = (size_t)h->rho.lmmaxvr * h->rho.nrmtmax * h->st.natmtot;
+  const size_t n = (size_t)h->rho.lmmaxvr * h->rho.nrmtmax * rho_atoms(h);
   if (magmt) CUDA_TRY(cudaMemcpyAsync(magmt, h->rho.magmt, sizeof(double) * n, cudaMemcpyDeviceToHost, h->stream));
   if (reset) CUDA_TRY(cudaMemsetAsync(h->rho.magmt, 0, sizeof(double) * n, h->stream));
   CUDA_TRY(cudaStreamSynchronize(h->stream));
@@ -795,7 +806,7 @@ int excfv_get_rhomt(excfv_handle* h, double* rhomt, int32_t reset) {
     return EXCFV_ERR_STATE;
   }
   DeviceGuard g(h->device);
-  const size_t n = (size_t)h->rho.lmmaxvr * h->rho.nrmtmax * h->st.natmtot;
+  const size_t n = (size_t)h->rho.lmmaxvr * h->rho.nrmtmax * rho_atoms(h);
   if (rhomt) CUDA_TRY(cudaMemcpyAsync(rhomt, h->rho.rhomt, sizeof(double) * n, cudaMemcpyDeviceToHost, h->stream));
   if (reset) CUDA_TRY(cudaMemsetAsync(h->rho.rhomt, 0, sizeof(double) * n, h->stream));
   CUDA_TRY(cudaStreamSynchronize(h->stream));

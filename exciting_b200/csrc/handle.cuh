@@ -59,13 +59,20 @@ struct DevStatic {
 // excfv_set_static can change them.
 struct Basis {
   int natmtot = 0, nspecies = 0, lmaxapw = 0, apwordmax = 0, maxaa = 0;
+  int nlomax = 0, maxnlo = 0, nlotot = 0, nstfv = 0;
   Basis() = default;
   explicit Basis(const DevStatic& st)
-      : natmtot(st.natmtot), nspecies(st.nspecies), lmaxapw(st.lmaxapw), apwordmax(st.apwordmax), maxaa(st.maxaa) {}
+      : natmtot(st.natmtot), nspecies(st.nspecies), lmaxapw(st.lmaxapw), apwordmax(st.apwordmax), maxaa(st.maxaa),
+        nlomax(st.nlomax), maxnlo(st.maxnlo), nlotot(st.nlotot), nstfv(st.nstfv) {}
   // whether arrays of these sizes have room for those of b
   bool holds(const Basis& b) const {
     return b.natmtot <= natmtot && b.nspecies <= nspecies && b.lmaxapw <= lmaxapw && b.apwordmax <= apwordmax &&
            b.maxaa <= maxaa;
+  }
+  // whether per-atom data made for these sizes still fits b's indexing
+  bool serves(const Basis& b) const {
+    return b.natmtot <= natmtot && b.nspecies <= nspecies && b.nstfv <= nstfv && b.apwordmax == apwordmax &&
+           b.maxaa == maxaa && b.nlomax == nlomax && b.maxnlo == maxnlo && b.nlotot == nlotot;
   }
 };
 
@@ -126,6 +133,7 @@ struct Workspace {
 // radial mesh, the SHT matrices, the rhomt accumulator, coefficient scratch.
 struct DevRho {
   bool ready = false;
+  Basis basis;  // at excfv_set_rho
   int lmaxvr = 0, lmmaxvr = 0, lradstep = 1, nrmtmax = 0, nrcmax = 0;
   size_t ncoef = 0;
   int* nrmt = nullptr;
@@ -159,6 +167,7 @@ struct DevRho {
 // interstitial field over the whole grid, scratch.
 struct DevSV {
   bool ready = false;
+  Basis basis;  // at excfv_set_bfield[_nc]
   bool nc = false;        // non-collinear field (ndmag = 3): one solve of order 2 nstfv
   bool so = false;        // spin-orbit terms in the blocks: alpha's alo = loa^H, else loa^T
   int ngrid[3] = {0, 0, 0};

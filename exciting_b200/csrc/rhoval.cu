@@ -513,6 +513,7 @@ int stage_set_rho(excfv_handle* h, const excfv_rhoset* r) {
     free_rho(d);
     return rc;
   }
+  d.basis = Basis(st);
   d.ready = true;
   return EXCFV_OK;
 }

@@ -298,6 +298,7 @@ int stage_set_bfield(excfv_handle* h, const excfv_bfield* b) {
     return rc;
   }
   for (int d = 0; d < 3; ++d) v.ngrid[d] = b->ngrid[d];
+  v.basis = Basis(st);
   v.ready = true;
   return EXCFV_OK;
 }
@@ -423,6 +424,7 @@ int stage_set_bfield_nc(excfv_handle* h, const excfv_bfield_nc* b) {
   for (int d = 0; d < 3; ++d) v.ngrid[d] = b->ngrid[d];
   v.nc = true;
   v.so = b->spinorb != 0;
+  v.basis = Basis(st);
   v.ready = true;
   return EXCFV_OK;
 }

@@ -231,7 +231,10 @@ typedef struct excfv_rhoset {
   const double* rfshtvr;   /* (lmmaxvr, lmmaxvr) */
 } excfv_rhoset;
 
-/* Uploads the rhovalk data and zeroes the handle's rhomt accumulator. */
+/* Uploads the rhovalk data and zeroes the handle's rhomt accumulator.  The data
+ * serve until excfv_set_static changes the basis (more atoms, species or states,
+ * other array dimensions): the density calls then return EXCFV_ERR_STATE until
+ * excfv_set_rho is called again. */
 int excfv_set_rho(excfv_handle* h, const excfv_rhoset* r);
 /* rhovalk (src/rhovalk.f90:13) for the spin-unpolarised ground state without
  * second-variational vectors: the k-point's muffin-tin valence density is
@@ -322,7 +325,8 @@ typedef struct excfv_bfield {
 
 /* Builds mt_hscf%alpha (mt_pot of the field, hmlint.f90:88-108; beta = -alpha)
  * and the interstitial field bir = (bxcir + birconst) cfunir in Fourier space
- * on the device. */
+ * on the device.  To be called again after an excfv_set_static that changes the
+ * basis, as excfv_set_rho. */
 int excfv_set_bfield(excfv_handle* h, const excfv_bfield* b);
 /* The non-collinear field (ndmag = 3: a field with x or y parts, or spin-orbit
  * coupling, init0.f90:190-203) of seceqnsv on its default path.  Host

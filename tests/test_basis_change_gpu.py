@@ -3,17 +3,20 @@
 What a handle keeps between calls is dimensioned by the basis that it was made for.
 A cell with more atoms and a larger lmaxapw, but fewer G+k vectors in arrays of the
 same leading dimension, needs larger matching-coefficient arrays than the workspace
-of the cell before had; single k-points and batches must get them.  Bounds as for the path's other cells.
+of the cell before had; single k-points and batches must get them.  The density's and
+the second variation's data are refused in a basis that they do not fit, and serve on
+in one that they do.  Bounds as for the path's other cells.
 """
 import numpy as np
 import pytest
 
 from exciting_b200 import synthetic as syn
 from exciting_b200.fv import FirstVariational
-from exciting_b200.lib import EXCFV_PREC_FP64, EXCFV_PREC_MIXED
-from oracle import fvref
+from exciting_b200.lib import EXCFV_PREC_FP64, EXCFV_PREC_MIXED, ExcfvError
+from oracle import fvref, rhoval
 
 pytestmark = pytest.mark.gpu
+EXCFV_ERR_STATE = -5
 
 
 def _solved(shape, ngkmax, **kw):
@@ -48,3 +51,37 @@ def test_workspaces_follow_the_basis(prec, etol, rtol):
             assert np.all(info == 0)
             for w, _ in outs:
                 assert np.abs(w - refs[0][2]).max() < etol
+
+
+def test_density_and_field_data_follow_the_basis():
+    lmaxvr, wocc = 2, np.array([1.0, 0.5, 0.0, 0.25, 0.75, 0.0, 0.0, 1.5])
+    zb, _, _, rf = rhoval.sht_matrices(lmaxvr)
+
+    def cell(nst):
+        p = syn.make_problem("diamond2", ngk=60, nstfv=nst, lmaxapw=4)
+        rad = syn.make_radial(p.static, nrmt=40, lmaxvr=lmaxvr)
+        X = fvref.seceqn(p.static, p.kpts[0])[1]
+        return p.static, p.kpts[0], rad, X
+
+    with FirstVariational(0) as fv:
+        for nst, fits in ((5, True), (8, False), (8, True), (4, True)):
+            st, kp, rad, X = cell(nst)
+            fv.set_static(st)
+            if nst == 5 or (nst == 8 and fits):
+                fv.set_rho(rad, lmaxvr, 1, zb, rf)
+                ng, _, c = syn.make_interstitial_real(st)
+                fv.set_bfield(rad, np.ones(((lmaxvr + 1) ** 2, 40, st.natmtot), order="F"), np.zeros(st.natmtot), ng,
+                              np.zeros(c.shape[0]), c, 0.002)
+            if fits:
+                fv.rhovalk(kp, X, wocc[:nst])
+                got = fv.rhomt(reset=True)
+                ref = rhoval.rhovalk(st, rad, 1, lmaxvr, kp.ngp, fvref.match(st, kp), X, wocc[:nst], 1e-8, zb, rf)
+                assert np.abs(got - ref).max() < 1e-12 * np.abs(ref).max()
+                fv.seceqnsv(kp, np.arange(nst) * 0.1, X)
+                continue
+            for call in (lambda: fv.rhovalk(kp, X, wocc[:nst]),
+                         lambda: fv.rhovalk_sv(kp, X, np.eye(2 * nst), np.ones(2 * nst)),
+                         lambda: fv.seceqnsv(kp, np.arange(nst) * 0.1, X)):
+                with pytest.raises(ExcfvError) as e:
+                    call()
+                assert e.value.code == EXCFV_ERR_STATE

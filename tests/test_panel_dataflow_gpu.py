@@ -9,11 +9,14 @@ Orders where the panels' shape changes on 148 SMs, in FP64 and in complex64 stor
               become resident while the panels go on (complex64: from 2240);
   3201        owners with two chunks of rows, the last owner with one, and a last
               block of one row.
+Two lanes of a batch have 74 SMs each, which is enough for the dataflow form up to
+order 1024: orders 664 to 964 on two lanes at once.
 Bounds as for the path's other orders.  Above 2000 the reference is a spectrum that
 the matrix is built with, instead of a minute of ZHEGVX.
 """
 import numpy as np
 import pytest
+from torch.profiler import ProfilerActivity, profile
 
 from exciting_b200 import synthetic as syn
 from exciting_b200.fv import FirstVariational
@@ -60,3 +63,25 @@ def test_orders(prec, n):
             assert np.abs(w - w_ref).max() < (1e-8 if mixed else 1e-10)
             assert fvref.residuals(h, o, w, x).max() < (1e-7 if mixed else 1e-13)
             assert fvref.o_orthonormality(o, x) < (1e-9 if mixed else 1e-11)
+
+
+@pytest.mark.parametrize("prec", [EXCFV_PREC_FP64, EXCFV_PREC_MIXED])
+def test_two_lanes(prec):
+    mixed = prec == EXCFV_PREC_MIXED
+    p = syn.make_problem("cubic8", nk=4, ngk_range=(820, 900) if mixed else (600, 900), nstfv=12, lmaxapw=6)
+    refs = []
+    for kp in p.kpts:
+        H, O = fvref.hamiltonandoverlapsetup(p.static, kp, fvref.match(p.static, kp))
+        refs.append((H, O, fvref.solvewithlapack(H, O, p.static.nstfv, p.static.evaltol, lwork=-1)[0]))
+    with FirstVariational(0, precision=prec) as fv:
+        fv.set_static(p.static)
+        fv.set_lanes(2)
+        with profile(activities=[ProfilerActivity.CUDA]) as prof:
+            runs = [fv.seceqn_batched(p.kpts, p.nmatmax) for _ in range(3)]
+    names = {e.key for e in prof.key_averages()}
+    assert any("k_tridiag_flow" in n for n in names) and not any("k_tridiag_panel" in n for n in names)
+    for outs, info in runs:
+        assert np.all(info == 0)
+        for (w, x), kp, (H, O, w_ref) in zip(outs, p.kpts, refs):
+            assert np.abs(w - w_ref).max() < (1e-8 if mixed else 1e-10)
+            assert fvref.residuals(H, O, w, x[:kp.nmat]).max() < (1e-7 if mixed else 1e-13)

@@ -1315,7 +1315,10 @@ static void group_segments(excfv_handle* h, const BatchArgs& b, int L, std::vect
 // Lanes of a batch when the caller has chosen none.  Orders that the cluster
 // kernel reduces alone in clusters of 8 have no cooperative panels to share the
 // SMs out to: up to 32 lanes, all k-points of most batches at once (28 k-points of
-// order ~300: 8 lanes 10.5 ms, 16 8.9, 28 6.1).  A lane's workspace is sized by the
+// order ~300: 8 lanes 10.5 ms, 16 8.9, 28 6.1).  Larger orders get 8, whatever their
+// number: measured on 12 k-points of order ~2050 in the precision form, 8 lanes take
+// 140 ms, 6 136 (two even waves) and 12 128, so this is not the best count there;
+// excfv_autotune_lanes finds it.  A lane's workspace is sized by the
 // caller's nmatmax, whatever the batch's orders: more than 8 lanes only while all of
 // them take at most a quarter of the memory that is free or already theirs.
 static int default_lanes(excfv_handle* h, const BatchArgs& b, int nmax) {

@@ -6,8 +6,9 @@
 // NBT columns of a panel, then one GEMM applies the rank-2*NBT update
 // C22 -= [V W] [W V]^H to the lower triangle of the trailing matrix (the only
 // part the reduction reads).  A handle with the whole GPU runs its panels as a
-// dataflow between thread blocks (tridiag_flow.cu); the kernel here, for the lanes
-// of a batch and as the fallback, costs two grid-wide barriers per column:
+// dataflow between thread blocks (tridiag_flow.cu), and so do two lanes of a batch up
+// to order 1024, whose 74 SMs hold that form's roles; the kernel here, for the lanes
+// of all other batches and as the fallback, costs two grid-wide barriers per column:
 //
 //   phase 1 (row owners)  finish W(:, i-1); update column c with the panel's
 //                         previous reflectors; partial |x|^2 for the norm
@@ -64,7 +65,7 @@ constexpr size_t panel_smem_bytes() {
 // Barrier of the TT consumer threads (named barrier 1; the producer warp does not take part).
 __device__ __forceinline__ void csync() { asm volatile("bar.sync 1, %0;" ::"n"(TT) : "memory"); }
 
-// Grid barrier on a monotonic arrival counter (zeroed before each launch):
+// Grid barrier on a monotonic arrival counter (zeroed before each reduction):
 // barrier number e completes when the counter reaches e * gridDim.x (plus
 // `planted`, nonzero only when a test arms a target nothing reaches).
 // Returns false when it timed out (here or in another CTA).
@@ -295,7 +296,7 @@ __global__ void __launch_bounds__(TT + 32, 1)
     const long long ntri = (long long)nt * (nt + 1) / 2;
     const long long t_beg = ntri * bid / G, t_end = ntri * (bid + 1) / G;
     constexpr int BPT = 64 / R::BC;    // TMA tiles (boxes) per 64-column tile
-      const int rg = tid & 15, cq = tid >> 4;
+    const int rg = tid & 15, cq = tid >> 4;
     double vav_re = 0.0, vav_im = 0.0;
     if (tid == 0) {
       const cplx alpha = ldT(C + (c + 1) + ld * c);

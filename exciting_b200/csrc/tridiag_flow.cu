@@ -41,10 +41,14 @@
 // wait of the launch has given up (status[ST_BARRIER]); all threads of a block then
 // leave at their next block barrier, which carries the decision.
 //
-// Measured against the barrier form (panels of one solve, cluster tail apart):
-// FP64 order 715 1.36 -> 0.75 ms, 1964 17.8 -> 9.7 ms, 5028 112 -> 90 ms;
-// complex64 order 1901 13.3 -> 6.8 ms.  A column takes 5.8 us at order 700, 7 at
-// 1400 and 10 at 1964, where a worker's tiles no longer all fit its ring.
+// Measured against the barrier form over the same columns (all panels of one solve,
+// the last 320 columns and the updates apart): FP64 order 715 4.15 -> 2.45 ms, 1964
+// 19.3 -> 11.6 ms; complex64 order 1901 17.8 -> 10.2 ms.  A column takes 6.0 us at
+// order 700, 6.7 at 1450, 7.4 at 1600, from where a worker's tiles no longer all fit
+// its ring, and 10.2 at 1964 (barrier form 10, 13.5, 13.5 and 14.8).  Of order 5028
+// the columns below 3136 go from 39.0 to 29.6 ms; those above, with two chunks per
+// owner and every tile from HBM, are slower than the barrier form's since that got
+// its present inner loop (69.2 against 58.9 ms).
 #include "tridiag_dev.cuh"
 
 namespace {

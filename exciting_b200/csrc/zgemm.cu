@@ -497,7 +497,10 @@ int zgemm(cudaStream_t s, int opA, int opB, const ZgemmArgs& a_in) {
   // time: rounds of CTAs over the SMs times a CTA's clocks (tile^2 / 16 per unit
   // of K, a tenth more for 32 x 32 tiles, which load twice as much per product,
   // plus a start of 3000), and for split K the reduction's launch and traffic.
-  // A large product always gets 64 x 64 tiles and one piece.  Products in place
+  // A large product always gets 64 x 64 tiles and one piece.  A lane of a batch
+  // counts all SMs too, not its share: its neighbours are seldom in a product at the
+  // same time (12 k-points of order ~2050 on 8 lanes 140 ms, with the share 144; 28 of
+  // order ~300 on 28 lanes 5.2 ms, with the share 5.4).  Products in place
   // (a panel overwritten by its own product) need one CTA per column of tiles:
   // 64-row tiles, no pieces.
   a.splitk = 1;

@@ -6,8 +6,8 @@
 // NBT columns of a panel, then one GEMM applies the rank-2*NBT update
 // C22 -= [V W] [W V]^H to the lower triangle of the trailing matrix (the only
 // part the reduction reads).  A handle with the whole GPU runs its panels as a
-// dataflow between thread blocks (tridiag_flow.cu), and so do two lanes of a batch up
-// to order 1024, whose 74 SMs hold that form's roles; the kernel here, for the lanes
+// dataflow between thread blocks (tridiag_flow.cu), as do two lanes of a batch from
+// order 1024 down, whose 74 SMs hold that form's roles; the kernel here, for the lanes
 // of all other batches and as the fallback, costs two grid-wide barriers per column:
 //
 //   phase 1 (row owners)  finish W(:, i-1); update column c with the panel's

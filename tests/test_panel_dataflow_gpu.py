@@ -9,7 +9,7 @@ Orders where the panels' shape changes on 148 SMs, in FP64 and in complex64 stor
               become resident while the panels go on (complex64: from 2240);
   3201        owners with two chunks of rows, the last owner with one, and a last
               block of one row.
-Two lanes of a batch have 74 SMs each, which is enough for the dataflow form up to
+Two lanes of a batch have 74 SMs each, enough for the dataflow form of blocks up to
 order 1024: orders 664 to 964 on two lanes at once.
 Bounds as for the path's other orders.  Above 2000 the reference is a spectrum that
 the matrix is built with, instead of a minute of ZHEGVX.

@@ -683,7 +683,7 @@ static int check_sv(excfv_handle* h, int ngp, int ngkmax, int nmatmax) {
     excfv_set_error("excfv_set_static and excfv_set_bfield must be called first");
     return EXCFV_ERR_STATE;
   }
-  if (!h->sv.basis.serves(Basis(h->st))) {
+  if (!h->sv.basis.serves(Basis(h->st)) || h->sv.basis.maxaa != h->st.maxaa) {
     excfv_set_error("excfv_set_bfield must be called again: excfv_set_static has changed the basis");
     return EXCFV_ERR_STATE;
   }

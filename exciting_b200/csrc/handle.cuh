@@ -72,7 +72,7 @@ struct Basis {
   // whether per-atom data made for these sizes still fits b's indexing
   bool serves(const Basis& b) const {
     return b.natmtot <= natmtot && b.nspecies <= nspecies && b.nstfv <= nstfv && b.apwordmax == apwordmax &&
-           b.maxaa == maxaa && b.nlomax == nlomax && b.maxnlo == maxnlo && b.nlotot == nlotot;
+           b.nlomax == nlomax && b.maxnlo == maxnlo && b.nlotot == nlotot;
   }
 };
 

@@ -37,22 +37,6 @@ int dalloc(T** p, size_t count) {
 }
 
 template <typename T>
-int upload(T** p, const void* host, size_t count) {
-  int rc = dalloc(p, count);
-  if (rc) return rc;
-  if (host) {
-    cudaError_t e = cudaMemcpy(*p, host, count * sizeof(T), cudaMemcpyHostToDevice);
-    if (e != cudaSuccess) {
-      excfv_set_error("upload: %s", cudaGetErrorString(e));
-      return EXCFV_ERR_CUDA;
-    }
-  } else {
-    cudaMemset(*p, 0, count * sizeof(T));
-  }
-  return EXCFV_OK;
-}
-
-template <typename T>
 void dfree(T*& p) {
   if (p) cudaFree(p);
   p = nullptr;
@@ -113,14 +97,18 @@ void excfv_set_error(const char* fmt, ...) {
   va_end(ap);
 }
 
-void free_static(DevStatic& st) {
-  dfree(st.idxis); dfree(st.rmt); dfree(st.apword); dfree(st.flist); dfree(st.fofl);
-  dfree(st.lo_atom); dfree(st.lo_local); dfree(st.lo_first); dfree(st.lo_lm); dfree(st.lo_ilo);
-  dfree(st.aa); dfree(st.loa); dfree(st.lolo); dfree(st.oalo); dfree(st.ololo); dfree(st.h1aa);
-  dfree(st.ivg); dfree(st.ivgig); dfree(st.veffig); dfree(st.xig); dfree(st.cfunig);
-  dfree(st.m2effig); dfree(st.zdinv);
+// forgets the arrays but keeps their memory for the next setting
+static void clear_static(DevStatic& st) {
   dfree(st.vgc); dfree(st.atposc); dfree(st.gkcount);
-  st.have_lattice = false;
+  const Block keep = st.block;
+  st = DevStatic();
+  st.block = keep;
+}
+
+void free_static(DevStatic& st) {
+  clear_static(st);
+  if (st.block.base) cudaFree(st.block.base);
+  st.block = Block();
 }
 
 void free_workspace(Workspace& ws) {
@@ -151,7 +139,7 @@ int handle_scratch(excfv_handle* h, size_t bytes, void** p) {
 int stage_set_static(excfv_handle* h, const excfv_static* s) {
   DevStatic& st = h->st;
   h->static_gen++;
-  free_static(st);
+  clear_static(st);
   h->have_static = false;
   if (!s || s->natmtot <= 0 || s->nspecies <= 0 || s->lmaxapw < 0 || s->apwordmax <= 0 ||
       s->maxaa <= 0 || s->ngvec <= 0 || s->ngrtot < s->ngvec || s->nstfv <= 0 || !s->idxis ||
@@ -286,48 +274,49 @@ int stage_set_static(excfv_handle* h, const excfv_static* s) {
       for (int ilo = 0; ilo < s->nlorb[is] && ilo < st.nlomax; ++ilo)
         st.h_lorbl[ilo + (size_t)std::max(1, st.nlomax) * is] = s->lorbl[ilo + (size_t)st.nlomax * is];
     }
-  if ((rc = upload(&st.idxis, idxis.data(), na))) return rc;
-  if ((rc = upload(&st.rmt, s->rmt, ns))) return rc;
-  if ((rc = upload(&st.apword, s->apword, (size_t)L1 * ns))) return rc;
-  if ((rc = upload(&st.flist, flist.data(), flist.size()))) return rc;
-  if ((rc = upload(&st.fofl, fofl.data(), fofl.size()))) return rc;
-  if ((rc = upload(&st.lo_atom, lo_atom.data(), lo_atom.size()))) return rc;
-  if ((rc = upload(&st.lo_local, lo_local.data(), lo_local.size()))) return rc;
-  std::vector<int> lo_first(na, -1);
-  for (int a = 0; a < na && a < (int)st.h_lo_first.size(); ++a) lo_first[a] = st.h_lo_first[a];
-  if ((rc = upload(&st.lo_first, lo_first.data(), lo_first.size()))) return rc;
-  if ((rc = upload(&st.lo_lm, lo_lm.data(), lo_lm.size()))) return rc;
-  if ((rc = upload(&st.lo_ilo, lo_ilo.data(), lo_ilo.size()))) return rc;
-  if ((rc = upload(&st.aa, s->aa, (size_t)st.maxaa * st.maxaa * na))) return rc;
-  if ((rc = upload(&st.loa, st.nlotot ? s->loa : nullptr, maxnlo1 * st.maxaa * na))) return rc;
-  if ((rc = upload(&st.lolo, st.nlotot ? s->lolo : nullptr, maxnlo1 * maxnlo1 * na))) return rc;
-  // upload(nullptr) zero-fills: a NULL aa / loa / lolo waits for excfv_hmlint
-  if ((rc = upload(&st.oalo, oalo.data(), noalo))) return rc;
-  if ((rc = upload(&st.ololo, ololo.data(), nololo))) return rc;
-  if (st.have_h1aa && (rc = upload(&st.h1aa, s->h1aa, nh1))) return rc;
-  if ((rc = upload(&st.ivg, s->ivg, (size_t)3 * st.ngrtot))) return rc;
-  if ((rc = upload(&st.ivgig, s->ivgig, nbox))) return rc;
-  if ((rc = upload(&st.veffig, s->veffig, st.ngvec))) return rc;
   const double* xsrc = (st.vrel != 0) ? s->meffig : s->cfunig;
   if (!xsrc) {
     excfv_set_error("excfv_set_static: meffig required when valence_relativity != 0");
     return EXCFV_ERR_ARG;
   }
-  if ((rc = upload(&st.xig, xsrc, st.ngvec))) return rc;
-  if ((rc = upload(&st.cfunig, s->cfunig, st.ngvec))) return rc;
   if (st.h1on && !s->m2effig) {
     excfv_set_error("excfv_set_static: m2effig required when h1on");
     return EXCFV_ERR_ARG;
   }
-  if ((rc = upload(&st.m2effig, st.h1on ? s->m2effig : nullptr, st.ngvec))) return rc;
-  if ((rc = dalloc(&st.zdinv, (size_t)st.apwordmax * st.apwordmax * L1 * na))) return rc;
+  std::vector<int> lo_first(na, -1);
+  for (int a = 0; a < na && a < (int)st.h_lo_first.size(); ++a) lo_first[a] = st.h_lo_first[a];
   double *d_spr = nullptr, *d_apwfr = nullptr;
-  if ((rc = upload(&d_spr, s->sprwin, (size_t)st.npmatch * ns))) return rc;
-  if ((rc = upload(&d_apwfr, s->apwfrwin, (size_t)st.npmatch * st.apwordmax * L1 * na))) return rc;
+  rc = set_arrays(st.block, h->stream, [&](auto&& put) {
+    put(&st.idxis, idxis.data(), na);
+    put(&st.rmt, s->rmt, ns);
+    put(&st.apword, s->apword, (size_t)L1 * ns);
+    put(&st.flist, flist.data(), flist.size());
+    put(&st.fofl, fofl.data(), fofl.size());
+    put(&st.lo_atom, lo_atom.data(), lo_atom.size());
+    put(&st.lo_local, lo_local.data(), lo_local.size());
+    put(&st.lo_first, lo_first.data(), lo_first.size());
+    put(&st.lo_lm, lo_lm.data(), lo_lm.size());
+    put(&st.lo_ilo, lo_ilo.data(), lo_ilo.size());
+    // zeros: a NULL aa / loa / lolo waits for excfv_hmlint, as h1aa does with h1on
+    put(&st.aa, s->aa, (size_t)st.maxaa * st.maxaa * na);
+    put(&st.loa, st.nlotot ? s->loa : nullptr, maxnlo1 * st.maxaa * na);
+    put(&st.lolo, st.nlotot ? s->lolo : nullptr, maxnlo1 * maxnlo1 * na);
+    put(&st.oalo, oalo.data(), noalo);
+    put(&st.ololo, ololo.data(), nololo);
+    if (st.h1on || st.have_h1aa) put(&st.h1aa, st.have_h1aa ? s->h1aa : nullptr, nh1);
+    put(&st.ivg, s->ivg, (size_t)3 * st.ngrtot);
+    put(&st.ivgig, s->ivgig, nbox);
+    put(&st.veffig, s->veffig, st.ngvec);
+    put(&st.xig, xsrc, st.ngvec);
+    put(&st.cfunig, s->cfunig, st.ngvec);
+    put(&st.m2effig, st.h1on ? s->m2effig : nullptr, st.ngvec);
+    put(&st.zdinv, (const void*)nullptr, (size_t)st.apwordmax * st.apwordmax * L1 * na);
+    put(&d_spr, s->sprwin, (size_t)st.npmatch * ns);
+    put(&d_apwfr, s->apwfrwin, (size_t)st.npmatch * st.apwordmax * L1 * na);
+  });
+  if (rc) return rc;
   rc = match_compute_zdinv(st, d_spr, d_apwfr, h->stream);
-  cudaStreamSynchronize(h->stream);
-  cudaFree(d_spr);
-  cudaFree(d_apwfr);
+  if (cudaStreamSynchronize(h->stream) != cudaSuccess && rc == EXCFV_OK) rc = EXCFV_ERR_CUDA;
   if (rc) return rc;
   h->have_static = true;
   return EXCFV_OK;

@@ -513,10 +513,6 @@ static int mt_build(excfv_handle* h, const excfv_mtrad* r, const double* pot, bo
     return EXCFV_ERR_ARG;
   }
   if (!pot) pot = r->veffmt;
-  if (olp && st.h1on && !st.h1aa) {
-    CUDA_TRY(cudaMalloc(&st.h1aa, sizeof(double) * st.apwordmax * st.apwordmax * (st.lmaxapw + 1) * st.natmtot));
-    CUDA_TRY(cudaMemset(st.h1aa, 0, sizeof(double) * st.apwordmax * st.apwordmax * (st.lmaxapw + 1) * st.natmtot));
-  }
   cudaStream_t s = h->stream;
   const int lmvr = (r->lmaxvr + 1) * (r->lmaxvr + 1);
   const int nlomax = std::max(st.nlomax, 1);

@@ -417,29 +417,20 @@ __global__ void k_rho_esv(int n, int spin, const cplx* evecsv, double epsocc, cp
   esv[t] = v;
 }
 
-template <typename T>
-int dup(T** d, const T* h, size_t n) {
-  *d = nullptr;
-  if (n == 0) n = 1;
-  CUDA_TRY(cudaMalloc(d, sizeof(T) * n));
-  if (h) CUDA_TRY(cudaMemcpy(*d, h, sizeof(T) * n, cudaMemcpyHostToDevice));
-  else CUDA_TRY(cudaMemset(*d, 0, sizeof(T) * n));
-  return EXCFV_OK;
-}
-
 }  // namespace
 
 void free_rho(DevRho& r) {
-  for (void* p : {(void*)r.nrmt, (void*)r.ucoarse, (void*)r.vcoarse, (void*)r.zb, (void*)r.rf, (void*)r.rhomt,
-                  (void*)r.coef, (void*)r.w, (void*)r.lo_first, (void*)r.lorbl, (void*)r.magmt, (void*)r.coef2,
-                  (void*)r.lo1, (void*)r.lo2, (void*)r.esv, (void*)r.magmt3, (void*)r.coef3, (void*)r.lo3, (void*)r.rtp, (void*)r.gang})
-    if (p) cudaFree(p);
+  if (r.block.base) cudaFree(r.block.base);
   r = DevRho();
 }
 
 int stage_set_rho(excfv_handle* h, const excfv_rhoset* r) {
   DevStatic& st = h->st;
-  free_rho(h->rho);
+  {  // forgets the data but keeps their memory
+    const Block keep = h->rho.block;
+    h->rho = DevRho();
+    h->rho.block = keep;
+  }
   if (r->lmaxvr < 0 || r->lmaxvr > RHO_LMAX || r->lmaxvr > st.lmaxapw || r->lradstep < 1 || r->nrmtmax < 1 ||
       !r->nrmt || !r->apwfr || !r->zbshtvr || !r->rfshtvr || (st.nlotot > 0 && !r->lofr)) {
     excfv_set_error("excfv_set_rho: lmaxvr must be 0..%d and <= lmaxapw, lradstep >= 1, arrays given", RHO_LMAX);
@@ -489,30 +480,31 @@ int stage_set_rho(excfv_handle* h, const excfv_rhoset* r) {
   const size_t L = d.lmmaxvr;
   d.ncoef = (size_t)st.apwordmax * L * std::max(st.nstfv, 1) * st.natmtot;
   d.gang_elems = rho_gang_elems((size_t)2 * std::max(st.nstfv, 1), L1 * st.apwordmax + nlomax, L, st.natmtot);
-  int rc;
-  if ((rc = dup(&d.nrmt, r->nrmt, st.nspecies)) || (rc = dup(&d.ucoarse, u.data(), u.size())) ||
-      (rc = dup(&d.vcoarse, v.data(), v.size())) ||
-      (rc = dup(&d.zb, reinterpret_cast<const cplx*>(r->zbshtvr), L * L)) || (rc = dup(&d.rf, r->rfshtvr, L * L)) ||
-      (rc = dup(&d.rhomt, (const double*)nullptr, L * r->nrmtmax * st.natmtot)) ||
-      (rc = dup(&d.coef, (const cplx*)nullptr, d.ncoef)) ||
-      (rc = dup(&d.w, (const double*)nullptr, (size_t)2 * std::max(st.nstfv, 1))) ||
-      (rc = dup(&d.lo_first, first.data(), st.natmtot)) ||
-      (rc = dup(&d.lorbl, st.h_lorbl.data(), st.h_lorbl.size())) ||
-      (rc = dup(&d.magmt, (const double*)nullptr, L * r->nrmtmax * st.natmtot)) ||
-      (rc = dup(&d.rtp, (const double*)nullptr, L * d.nrcmax * st.natmtot)) ||
-      (rc = dup(&d.gang, (const cplx*)nullptr, d.gang_elems)) ||
-      (rc = dup(&d.coef2, (const cplx*)nullptr, 2 * d.ncoef)) ||
-      (rc = dup(&d.lo1, (const cplx*)nullptr, (size_t)std::max(st.maxnlo, 1) * st.natmtot * std::max(st.nstfv, 1))) ||
-      (rc = dup(&d.lo2, (const cplx*)nullptr,
-                (size_t)2 * std::max(st.maxnlo, 1) * st.natmtot * std::max(st.nstfv, 1))) ||
-      (rc = dup(&d.esv, (const cplx*)nullptr, (size_t)2 * std::max(st.nstfv, 1) * std::max(st.nstfv, 1))) ||
-      (rc = dup(&d.magmt3, (const double*)nullptr, 3 * L * r->nrmtmax * st.natmtot)) ||
-      (rc = dup(&d.coef3, (const cplx*)nullptr, 2 * d.ncoef)) ||
-      (rc = dup(&d.lo3, (const cplx*)nullptr,
-                (size_t)2 * std::max(st.maxnlo, 1) * st.natmtot * std::max(st.nstfv, 1)))) {
-    free_rho(d);
-    return rc;
-  }
+  const size_t nst = std::max(st.nstfv, 1), nlo = (size_t)std::max(st.maxnlo, 1) * st.natmtot;
+  const int rc = set_arrays(d.block, h->stream, [&](auto&& put) {
+    put(&d.nrmt, r->nrmt, st.nspecies);
+    put(&d.ucoarse, u.data(), u.size());
+    put(&d.vcoarse, v.data(), v.size());
+    put(&d.zb, r->zbshtvr, L * L);
+    put(&d.rf, r->rfshtvr, L * L);
+    put(&d.lo_first, first.data(), st.natmtot);
+    put(&d.lorbl, st.h_lorbl.data(), st.h_lorbl.size());
+    put(&d.rhomt, nullptr, L * r->nrmtmax * st.natmtot);
+    put(&d.magmt, nullptr, L * r->nrmtmax * st.natmtot);
+    put(&d.magmt3, nullptr, 3 * L * r->nrmtmax * st.natmtot);
+    put(&d.w, nullptr, 2 * nst);
+    put(&d.rtp, nullptr, L * d.nrcmax * st.natmtot);
+    put(&d.gang, nullptr, d.gang_elems);
+    put(&d.coef, nullptr, d.ncoef);
+    put(&d.coef2, nullptr, 2 * d.ncoef);
+    put(&d.coef3, nullptr, 2 * d.ncoef);
+    put(&d.lo1, nullptr, nlo * nst);
+    put(&d.lo2, nullptr, 2 * nlo * nst);
+    put(&d.lo3, nullptr, 2 * nlo * nst);
+    put(&d.esv, nullptr, 2 * nst * nst);
+  });
+  if (rc) return rc;
+  CUDA_TRY(cudaStreamSynchronize(h->stream));
   d.basis = Basis(st);
   d.ready = true;
   return EXCFV_OK;
